@@ -328,7 +328,14 @@ struct Cell {
        shared memory, which the network code reloads instead of spilling */
     alignas(16) std::conditional_t<SHM == 4, double*, double[N]> y;
     typename Staging<Net, LUT, SHM, BS>::LU a; /* packed LU of the iteration matrix */
-    alignas(16) double rT[NR];
+    /* temperature part of the rates: an array of its own, not a member.  The
+       set-up call that fills it takes its address, and as a member it would
+       keep this whole object (state, weights, corrections, every control
+       word) in local memory: PRIMORDIAL then executed 2.9 times the local
+       loads and stores, and was 1.15 times slower (1,048,576 cells, FP32
+       LU: 135.9 ms at its best shape, 118.1 ms without, one 256-thread
+       block per SM; FP64 175.6 and 162.6 ms) */
+    double* rT;
     /* FP32 LU: the scale of species j is 2^sce[j] (kept as an exponent, the
        factors are formed only while the Jacobian and the solve run) */
     short sce[SCALED ? ND : 1];
@@ -883,8 +890,21 @@ __device__ __forceinline__ void bdf_run(const LaunchArgs& A)
     alignas(16) LUT lu_local[SHM == 1 ? 1 : C::NNZ];
     if constexpr (SHM == 0 || SHM == 4)
         c.yns = history;
-    if constexpr (SHM != 1)
+    if constexpr (SHM != 1) {
         c.a = lu_local;
+        /* The LU of a network of more than a few species stays in memory:
+           its constant indices would let the compiler spread it over
+           registers that it does not have, and spill around every phase
+           (PRIMORDIAL, 84 entries: 145 ms against 118 ms with FP32 factors,
+           206 against 163 ms in FP64).  Taking its address in an empty
+           statement keeps it an array.  The 506 FP32 factors of SYN64 are
+           the exception (446 against 465 ms; its FP64 factors 576 against
+           527 ms). */
+        if constexpr (C::NNZ > 16 && (sizeof(LUT) == 8 || C::NNZ <= 128))
+            asm volatile("" ::"l"(&lu_local[0]) : "memory");
+    }
+    alignas(16) double rates_local[C::NR];
+    c.rT = rates_local;
     int ph = PH_IDLE;
     int64_t cell = -1;
     bool write_y = false;
@@ -1043,8 +1063,8 @@ __device__ __forceinline__ void bdf_run(const LaunchArgs& A)
                     for (int j = 0; j < ND; ++j)
                         if (c.msk)
                             c.y[Net::dyn(j)] = c.yns[0][j];
-                    if (Net::NREA > 0)
-                        Net::rates_T(c.y, c.rT);
+                    if constexpr (Net::NREA > 0)
+                        Net::rates_T(c.y[Net::IDX_TGAS], c.rT);
                     c.ujac = true;
                     if (c.t < c.tstop) {
                         c.told = c.t;
@@ -1065,8 +1085,8 @@ __device__ __forceinline__ void bdf_run(const LaunchArgs& A)
                         for (int j = 0; j < ND; ++j)
                             c.eno[j] = A.ws[((int64_t)(MAXQ + 1) * ND + j) * stride + cell];
                     }
-                    if (Net::NREA > 0)
-                        Net::rates_T(c.y, c.rT);
+                    if constexpr (Net::NREA > 0)
+                        Net::rates_T(c.y[Net::IDX_TGAS], c.rT);
 #pragma unroll
                     for (int j = 0; j < ND; ++j)
                         c.yns[0][j] = c.y[Net::dyn(j)];

@@ -26,7 +26,7 @@ struct ov_net_rober_dense_none_lu2 {
   OV_HD static constexpr int frozen(int i) { return 0; }
   OV_HD static OV_INLINE void rhs(const double* y, const double* k, double* f) { ov_rober_dense_none_lu2_rhs(y, k, f); }
   static OV_INLINE __device__ void rates_k(const double*, const double*, double*) {}
-  static OV_INLINE __device__ void rates_T(const double*, double*) {}
+  static OV_INLINE __device__ void rates_T(double, double*) {}
   /* P = I - dt*beta*J on the dynamic block, packed CSC order */
   template <class T, class A> OV_HD static OV_INLINE void jac(const double* OV_RESTRICT y, const double* OV_RESTRICT k, double beta, double dt, A a) {
     (void)y; (void)k; (void)beta; (void)dt; (void)a;

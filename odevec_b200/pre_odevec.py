@@ -808,11 +808,14 @@ def emit_cuda_header(sysm: System) -> str:
     if net.rates:
         L.append("  static OV_INLINE __device__ void rates_k(const double* y, const double* r, double* k) "
                  "{ ov_rates_%s_k(y, %d, r, k); }" % (net.rates, n))
-        L.append("  static __device__ __noinline__ void rates_T(const double* y, double* r) "
-                 "{ ov_rates_%s_T(y[%d], r); }" % (net.rates, net.idx_tgas))
+        # a call: its arguments are the temperature by value and the rate array
+        # alone, since every array whose address it took would have to live
+        # in memory for the whole kernel
+        L.append("  static __device__ __noinline__ void rates_T(double Tgas, double* r) "
+                 "{ ov_rates_%s_T(Tgas, r); }" % net.rates)
     else:
         L.append("  static OV_INLINE __device__ void rates_k(const double*, const double*, double*) {}")
-        L.append("  static OV_INLINE __device__ void rates_T(const double*, double*) {}")
+        L.append("  static OV_INLINE __device__ void rates_T(double, double*) {}")
     L.append("  /* P = I - dt*beta*J on the dynamic block, packed CSC order */")
     src = _jac_source(sysm)
     L.append("  template <class T, class A> OV_HD static OV_INLINE void jac(const double* OV_RESTRICT y, "
