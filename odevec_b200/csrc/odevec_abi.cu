@@ -154,6 +154,8 @@ int find_net(const char* tag)
 
 }  // namespace
 
+constexpr int OV_RATE_TABS = 48; /* doubling sizes: never reached */
+
 struct odevec_solver {
     int net;
     int64_t max_cells;
@@ -181,6 +183,15 @@ struct odevec_solver {
     void* ord_temp;
     size_t ord_temp_bytes;
     const int32_t* ord_cur;
+    /* rate tables ([cells][reactions], networks with rate coefficients): the
+       last one is in use, of rate_cells cells; smaller ones before it stay
+       until odevec_close, since a captured graph may hold their address.
+       Each is at least twice the one before it.  rate_cur: that of the last
+       solve, or null (a continuation reuses it) */
+    int64_t rate_cells;
+    int rate_ntabs;
+    double* rate_tabs[OV_RATE_TABS];
+    double* rate_cur;
 };
 /* d_queue words: [0] the solve's work counter, [1] cells that failed with
    FP32 factors, [2] the FP64 re-solve's work counter */
@@ -188,6 +199,9 @@ struct odevec_solver {
    sort, and where a persistent grid holds (nearly) every cell at once
    (19k-57k lanes resident) there is no tail to shorten */
 constexpr int64_t OV_ORDER_MIN_CELLS = 32768;
+/* fewer cells evaluate their rates as they are set up (nearly all on the
+   launch's first trip, so with full warps) */
+constexpr int64_t OV_RATES_MIN_CELLS = 4096;
 
 namespace {
 /* sort keys of the visit order: the top 16 bits of t_stop - t (a
@@ -516,6 +530,41 @@ static int32_t visit_order(odevec_solver* s, int64_t ncells, const double* t, co
     return OV_API_OK;
 }
 
+/* The rate table of a solve of a network with rate coefficients: one kernel
+   evaluates the temperature part of every cell's rates with all lanes busy.
+   Evaluated in the solve kernel as each cell is set up, the same laws run
+   for the two or three lanes of a warp that take a cell at the same time.
+   Without a table (no room for it, a capture that would have to allocate it,
+   or few cells) the solve kernel evaluates them, with the same results. */
+static cudaError_t rate_table(odevec_solver* s, ov::LaunchArgs& a, ov::launch_fn fn, cudaStream_t st)
+{
+    a.rates = s->rate_cur = nullptr;
+    const int64_t nrea = g_nets[s->net].sizes[2];
+    if (nrea <= 0 || a.ncells < OV_RATES_MIN_CELLS)
+        return cudaSuccess;
+    if (s->rate_cells < a.ncells) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+            s->rate_ntabs >= OV_RATE_TABS) {
+            cudaGetLastError();
+            return cudaSuccess;
+        }
+        const int64_t cells = a.ncells > 2 * s->rate_cells ? a.ncells : 2 * s->rate_cells;
+        double* tab = nullptr;
+        if (cudaMalloc(&tab, sizeof(double) * (size_t)nrea * (size_t)cells) != cudaSuccess) {
+            cudaGetLastError();
+            return cudaSuccess;
+        }
+        s->rate_tabs[s->rate_ntabs++] = tab;
+        s->rate_cells = cells;
+    }
+    a.rates = s->rate_tabs[s->rate_ntabs - 1];
+    const cudaError_t e = fn(a, 1, 0, ov::STAGE_RATES, 0, 0, st);
+    if (e == cudaSuccess)
+        s->rate_cur = a.rates;
+    return e;
+}
+
 static int32_t solve_impl(odevec_solver* s, int64_t ncells, int64_t stride, double* y, double* t,
                           double* dt, const double* t_stop, const uint8_t* mask, int32_t* status,
                           int32_t* stats, double* ws, int32_t resume, void* stream, bool cont)
@@ -561,6 +610,7 @@ static int32_t solve_impl(odevec_solver* s, int64_t ncells, int64_t stride, doub
     a.save_y = a.save_t = a.save_dt = nullptr;
     a.yield = s->yield;
     a.order = nullptr;
+    a.rates = cont ? s->rate_cur : nullptr;
     cudaStream_t st = (cudaStream_t)stream;
     /* a continuation keeps the work counter (and the failure count) of the
        solve it continues */
@@ -622,7 +672,10 @@ static int32_t solve_impl(odevec_solver* s, int64_t ncells, int64_t stride, doub
         if (!a.status)
             a.status = s->fb_status;
     }
-    err = fn(a, o.group_size, lu, stage, o.block_threads, o.grid_blocks, st);
+    if (!cont)
+        err = rate_table(s, a, fn, st);
+    if (err == cudaSuccess)
+        err = fn(a, o.group_size, lu, stage, o.block_threads, o.grid_blocks, st);
     if (escalate && err == cudaSuccess) {
         int blocks = 0;
         cudaDeviceGetAttribute(&blocks, cudaDevAttrMultiProcessorCount, s->device);
@@ -792,6 +845,8 @@ int32_t odevec_close(odevec_solver* s)
     cudaFree(s->ord_keys);
     cudaFree(s->ord_vals);
     cudaFree(s->ord_temp);
+    for (int i = 0; i < s->rate_ntabs; ++i)
+        cudaFree(s->rate_tabs[i]);
     cudaFree(s->d_y);
     cudaFree(s->d_t);
     cudaFree(s->d_dt);
@@ -980,6 +1035,7 @@ extern "C" int32_t odevec_solve_noalloc(const char* network, const odevec_opts* 
     a.save_y = a.save_t = a.save_dt = nullptr;
     a.yield = nullptr;
     a.order = nullptr;
+    a.rates = nullptr;
     const NetEntry& e = g_nets[ni];
     const int lu = o.precision == OV_PREC_FP32_LU ? 1 : 0;
     ov::launch_fn fn = o.precision == OV_PREC_FP64 ? e.exact : e.fma;
@@ -1088,6 +1144,10 @@ extern "C" int32_t odevec_solve_many(const odevec_job* jobs, int32_t njobs, void
         const int32_t rc = visit_order(J.solver, J.ncells, J.t, J.t_stop, st, &a.order);
         if (rc)
             return rc;
+        const NetEntry& e = g_nets[J.solver->net];
+        err = rate_table(J.solver, a, prec == OV_PREC_FP64 ? e.exact : e.fma, st);
+        if (err != cudaSuccess)
+            return fail(OV_API_ECUDA, "odevec_solve_many: %s", cudaGetErrorString(err));
     }
     const int lu = prec == OV_PREC_FP32_LU ? 1 : 0;
     ov::multi_fn fn = prec == OV_PREC_FP64 ? m->exact : m->fma;

@@ -59,7 +59,15 @@ struct LaunchArgs {
        counter is cell order[q] (a permutation of 0..ncells-1), so cells are
        visited in that order; results do not depend on it */
     const int32_t* order;
+    /* networks with rate coefficients: if non-null, the temperature part of
+       every cell's rates, [ncells][NREA], filled by the rates kernel
+       (STAGE_RATES) earlier on the stream; null: each cell evaluates its
+       own as it is set up */
+    double* rates;
 };
+
+/* "staging" that fills LaunchArgs::rates instead of solving */
+constexpr int STAGE_RATES = -1;
 
 /* Several solves of different networks in one launch (the multi-network
    kernel): job j's launch arguments, the index of its network in the

@@ -255,7 +255,10 @@ class GpuBackend:
         return ode
 
     def bytes_needed(self, r: Request) -> float:
-        per_cell = 8 * (r.y0.shape[0] + 3 + self.S.workspace_doubles(r.network)) + 4 + 8 * 8
+        # state, times, workspace, status, statistics, and the solver's table
+        # of rate coefficients
+        per_cell = (8 * (r.y0.shape[0] + 3 + self.S.workspace_doubles(r.network)
+                         + self.S.network_info(r.network)["nrea"]) + 4 + 8 * 8)
         return float(per_cell * r.ncells)
 
     def admit(self, r: Request):

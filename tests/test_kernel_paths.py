@@ -1,0 +1,48 @@
+"""The solve kernels' size-dependent paths against the CPU oracle, bit for
+bit (fp64), at the sizes where a path starts, ends or changes."""
+import numpy as np
+import pytest
+
+from odevec_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _solver(S, wl, **kw):
+    kw.setdefault("precision", "fp64")
+    kw.setdefault("nvector", wl.group)
+    ode = S.Odevec(wl.network, RelativeTolerance=wl.rtol, AbsoluteTolerance=wl.atol, MinimalTimestep=wl.dt_min,
+                   raise_on_failure=False, **kw)
+    S.InitOdevec(ode)
+    return ode
+
+
+def _gpu(S, ode, wl, mask=None):
+    import torch
+    y = torch.tensor(wl.y, device="cuda")
+    t, dt = S.SolveODE(ode, torch.tensor(wl.t0, device="cuda"), torch.tensor(wl.dt0, device="cuda"),
+                       torch.tensor(wl.t_stop, device="cuda"), y, Mask=mask)
+    torch.cuda.synchronize()
+    return [a.cpu().numpy() for a in (y, t, dt, ode.status, ode.stats)]
+
+
+def _oracle(O, wl, group=None, **kw):
+    return O.solve(wl.network, wl.y, wl.t0, wl.dt0, wl.t_stop, wl.rtol, wl.atol, wl.dt_min,
+                   group=wl.group if group is None else group, **kw)
+
+
+def _same(g, o):
+    for name, a, b in zip(("y", "t", "dt", "status", "stats"), g, o):
+        assert np.array_equal(a, b), "%s differs in %d places" % (name, int(np.sum(np.asarray(a) != np.asarray(b))))
+
+
+def test_rate_table_sizes(gpu_lib, oracle):
+    """Solves below, at and above the size from which the rates come from a
+    table, on one solver whose table grows in between."""
+    wls = {n: W.primordial(ncells=n, seed=20 + n % 7) for n in (4095, 4096, 9001)}
+    ode = _solver(gpu_lib, wls[4096])
+    try:
+        for n in (4095, 4096, 9001, 4096):
+            _same(_gpu(gpu_lib, ode, wls[n]), _oracle(oracle, wls[n]))
+    finally:
+        gpu_lib.CloseOdevec(ode)
