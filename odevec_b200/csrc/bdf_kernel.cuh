@@ -119,6 +119,14 @@ static __constant__ double c_tau[6][4] = {
 __device__ __forceinline__ double tau(int order, int order2) { return c_tau[order][order2 - order + 1]; }
 __device__ __forceinline__ double conv_divisor(int order) { return c_tau[order][3]; }
 
+/* per order q: the smallest double x with sqrt(x) / tau(q,q) > 1 in double
+   arithmetic, i.e. whose rounded root exceeds tau(q,q).  The local error
+   test norm / tau > 1 (src/odevec.F90:402-404) then needs neither the root
+   nor the division: both are monotone, so comparing the norm's square with
+   this bound decides the same way for every input */
+static __constant__ double c_lte[6] = {0.0, 0x1.0000000000002p+2, 0x1.4400000000002p+4, 0x1.ae38e38e38e3cp+5,
+                                       0x1.b2071c71c71cbp+6, 0x1.776147ae147b0p+7};
+
 /* NaN and masked-out values never win a max (as the oracle's comparison loop) */
 __device__ __forceinline__ double max_operand(double v) { return v > -HUGE_VAL ? v : -HUGE_VAL; }
 
@@ -376,8 +384,19 @@ struct Cell {
         return wnorm(e, s);
     }
 
-    /* WeightedNorm2 of y_NS(:,:,col) for a runtime column */
-    __device__ __forceinline__ double wnorm_ns(int col) const
+    /* the square of wnorm(e): div_n of the sum of squares, before the root */
+    __device__ __forceinline__ double wnorm_sq(const double* e) const
+    {
+        double s = 0.0;
+#pragma unroll
+        for (int j = 0; j < ND; ++j)
+            s = s + e[j] * e[j] * w2[j];
+        s = s + fz_add;
+        return group_max<G>(msk ? div_n(s) : -HUGE_VAL);
+    }
+
+    /* the square of WeightedNorm2 of y_NS(:,:,col) for a runtime column */
+    __device__ __forceinline__ double wnorm_ns_sq(int col) const
     {
         double s = 0.0;
 #pragma unroll
@@ -386,8 +405,7 @@ struct Cell {
             s = s + e * e * w2[j];
         }
         s = s + fz_add;
-        double v = msk ? sqrt(div_n(s)) : -HUGE_VAL;
-        return group_max<G>(v);
+        return group_max<G>(msk ? div_n(s) : -HUGE_VAL);
     }
 
     /* CalcErrorWeightInvSquared (src/odevec.F90:706-716) */
@@ -497,44 +515,81 @@ struct Cell {
 
     /* CalcStepSizeOrder (src/odevec.F90:547-618); returns dt_scale.  The
        literals 1.3, 1.2, 1.4 and 1.1 are single precision in the reference.
-       The three candidate factors are independent: with per-cell control all
-       three are evaluated (the unused ones are discarded) with the
-       branch-free power, so their dependency chains interleave instead of
-       running one after another; a lockstep group (whose order is uniform)
-       skips the unused norms and their shuffle reductions.  Each kept value
-       is the same IEEE expression as in the reference. */
+
+       Of the three candidate factors (order - 1, same, + 1) only one is used:
+       the largest if it reaches 1.1, else the one of the same order.  Which
+       one that is follows from single-precision estimates (relative error
+       below 1e-4) unless two candidates, or the largest and 1.1, lie within
+       1e-3 of each other; then all are evaluated.  So a lane evaluates one
+       root, quotient and power instead of three, each kept value the same
+       IEEE expression as in the reference.  Bound by the chain of dependent
+       FP64 operations of a power (1,048,576 PRIMORDIAL cells with FP32
+       factors: 109.3 -> 107.4 ms; a lockstep group evaluated three powers one
+       after another). */
     __device__ __forceinline__ double step_size_order()
     {
         const int order = q;
-        const bool want_down = G == 1 || order != 1;
-        const bool want_up = G == 1 || !(order == MAXQ || nuo);
-        double d[ND];
+        const bool has_down = order != 1, has_up = !(order == MAXQ || nuo);
+        /* squared norms; a lockstep group (uniform order) skips unused ones */
+        const double x_down = G == 1 || has_down ? wnorm_ns_sq(order) : 0.0;
+        const double x_same = wnorm_sq(en);
+        double x_up = 0.0;
+        if (G == 1 || has_up) {
+            double d[ND];
 #pragma unroll
-        for (int j = 0; j < ND; ++j)
-            d[j] = en[j] - eno[j];
-        const double n_down = want_down ? wnorm_ns(order) / tau(order, order - 1) : 0.0;
-        const double n_same = wnorm(en) / tau(order, order);
-        const double n_up = want_up ? wnorm(d) / tau(order, order + 1) : 0.0;
-        const double p_down = ov_pow_sel(n_down, c_inv[order]);
-        const double p_same = ov_pow_sel(n_same, c_inv[order + 1]);
-        const double p_up = ov_pow_sel(n_up, c_inv[order + 2]);
-        const double down = order == 1 ? 0.0 : 1.0 / ((double)1.3f * p_down + 1e-6);
-        const double same = 1.0 / ((double)1.2f * p_same + 1e-6);
-        const double up = (order == MAXQ || nuo) ? 0.0 : 1.0 / ((double)1.4f * p_up + 1e-6);
-        int loc = 1;
-        double mx = down;
-        if (same > mx) { mx = same; loc = 2; }
-        if (up > mx) { mx = up; loc = 3; }
-        double s = mx;
-        if (s >= (double)1.1f) {
+            for (int j = 0; j < ND; ++j)
+                d[j] = en[j] - eno[j];
+            x_up = wnorm_sq(d);
+        }
+        /* candidate loc = 1, 2, 3: 1 / (c * (norm / tau)^(1/k) + 1e-6) */
+        auto factor = [&](int loc) {
+            const double x = loc == 1 ? x_down : (loc == 2 ? x_same : x_up);
+            const double cc = loc == 1 ? (double)1.3f : (loc == 2 ? (double)1.2f : (double)1.4f);
+            const double n = (x < 0.0 ? x : sqrt(x)) / c_tau[order][loc - 1];
+            return 1.0 / (cc * ov_pow_sel(n, c_inv[order + loc - 1]) + 1e-6);
+        };
+        auto estimate = [&](double x, float cc, int loc) {
+            const int hi = __double2hiint(x);
+            const float m = __int_as_float(0x3f800000 | ((hi & 0xfffff) << 3));
+            const float l = (float)((hi >> 20) - 1023) + __log2f(m);
+            return cc * exp2f((0.5f * l - __log2f((float)c_tau[order][loc - 1])) * (float)c_inv[order + loc - 1])
+                   + 1e-6f;
+        };
+        const float e_same = estimate(x_same, 1.2f, 2);
+        const float e_down = has_down ? estimate(x_down, 1.3f, 1) : HUGE_VALF;
+        const float e_up = has_up ? estimate(x_up, 1.4f, 3) : HUGE_VALF;
+        const float best = fminf(e_same, fminf(e_down, e_up));
+        const float near_best = best * 1.001f;
+        const bool one_best = (e_same <= near_best) + (e_down <= near_best) + (e_up <= near_best) == 1;
+        const bool below = best * 1.1f > 1.001f; /* the largest factor is below 1.1 */
+        const bool above = best * 1.1f < 0.999f;
+        /* infinities and NaN (a negative squared norm) take the full comparison */
+        const bool finite = x_same >= 0.0 && x_same < HUGE_VAL && (!has_down || (x_down >= 0.0 && x_down < HUGE_VAL))
+                            && (!has_up || (x_up >= 0.0 && x_up < HUGE_VAL));
+        const bool clear = finite && (below || (above && one_best));
+        int loc = 2;
+        if (clear && above)
+            loc = e_down <= near_best ? 1 : (e_up <= near_best ? 3 : 2);
+        double s = factor(loc);
+        bool big = above;
+        if (!clear) {
+            const double same = s;
+            const double down = has_down ? factor(1) : 0.0;
+            const double up = has_up ? factor(3) : 0.0;
+            loc = 1;
+            double mx = down;
+            if (same > mx) { mx = same; loc = 2; }
+            if (up > mx) { mx = up; loc = 3; }
+            big = mx >= (double)1.1f;
+            s = big ? mx : same;
+        }
+        if (big) {
             if (loc == 1) {
                 if (order != 1)
                     q = order - 1;
                 else
                     status = OV_ERR_ORDER;
-            } else if (loc == 2) {
-                s = same;
-            } else {
+            } else if (loc == 3) {
                 if (order != MAXQ) {
                     const double c = lcoef(order, order);
 #pragma unroll
@@ -544,8 +599,6 @@ struct Cell {
                 } else
                     status = OV_ERR_ORDER;
             }
-        } else {
-            s = same;
         }
         double upper;
         if (first) {
@@ -571,7 +624,7 @@ struct Cell {
             crate = fmax(0.2 * crate, rate_tmp);
         }
         const double r15 = 1.5 * crate;
-        const double crit = err * (1.0 < r15 ? 1.0 : r15) / conv_divisor(q);
+        const double crit = err * (1.0 < r15 ? 1.0 : r15);
         /* a NaN in den or in the weights (src/odevec.F90:645) makes its
            term and so the lane's sum of squares NaN: the entries are only
            scanned when that sum is NaN */
@@ -586,7 +639,8 @@ struct Cell {
             failed = true;
             return;
         }
-        if (crit < 1.0) {
+        /* crit / D < 1: the rounded quotient is below 1 exactly when crit < D */
+        if (crit < conv_divisor(q)) {
             converged = true;
             return;
         }
@@ -1284,9 +1338,9 @@ __device__ __forceinline__ void bdf_run(const LaunchArgs& A)
             } else if (converged) {
                 c.fc = 0;
                 /* local truncation error test (src/odevec.F90:400-455) */
-                const double error = c.wnorm(c.en) / tau(c.q, c.q);
+                const bool lte = c.wnorm_sq(c.en) >= c_lte[c.q];
                 c.weights(A.rtol, A.atol);
-                if (error > 1.0) {
+                if (lte) {
                     c.ltef++;
                     c.t = c.told;
                     if (c.fet >= 3) {

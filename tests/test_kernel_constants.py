@@ -1,0 +1,46 @@
+"""Constants of the CUDA kernel that stand for exact decisions of the
+reference's arithmetic."""
+import math
+import os
+import re
+
+import pytest
+
+CUH = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "odevec_b200", "csrc",
+                   "bdf_kernel.cuh")
+
+
+def _tau(order, order2):
+    """src/odevec.F90:1034-1054 with IEEE doubles"""
+    last = [0.0, 1.0, 1.0 / 3.0, 1.0 / 11.0, 1.0 / 50.0, 1.0 / 274.0, 1.0 / 1764.0]
+    fac = 1.0
+    for i in range(1, order + 1):
+        fac = fac * i
+    if order - 1 == order2:
+        return (order2 + 1.0) / fac
+    return (order2 + 1.0) / (fac * last[order])
+
+
+@pytest.mark.parametrize("q", [1, 2, 3, 4, 5])
+def test_local_error_bound(q):
+    """c_lte[q] is the smallest double x for which sqrt(x) / tau(q,q) > 1."""
+    text = open(CUH).read()
+    vals = re.search(r"c_lte\[6\] = \{([^}]*)\}", text).group(1).split(",")
+    x = float.fromhex(vals[q].strip())
+    tau = _tau(q, q)
+    assert math.sqrt(x) / tau > 1.0
+    assert not math.sqrt(math.nextafter(x, 0.0)) / tau > 1.0
+
+
+@pytest.mark.parametrize("q", [1, 2, 3, 4, 5])
+def test_convergence_quotient(q):
+    """a / D < 1 for the rounded quotient exactly when a < D, next to D."""
+    D = _tau(q, q) / (2.0 * (q + 2.0))
+    a = D
+    for _ in range(40):
+        assert (a / D < 1.0) == (a < D)
+        a = math.nextafter(a, 0.0)
+    a = D
+    for _ in range(40):
+        assert (a / D < 1.0) == (a < D)
+        a = math.nextafter(a, math.inf)
