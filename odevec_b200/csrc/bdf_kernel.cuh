@@ -130,6 +130,28 @@ static __constant__ double c_lte[6] = {0.0, 0x1.0000000000002p+2, 0x1.4400000000
 /* NaN and masked-out values never win a max (as the oracle's comparison loop) */
 __device__ __forceinline__ double max_operand(double v) { return v > -HUGE_VAL ? v : -HUGE_VAL; }
 
+/* Correctly rounded reciprocal of x in [2^-1000, 2^1000) whose significand is
+   not all ones: Newton's iteration from the hardware estimate, the last step
+   with the residual formed exactly by a fused multiply-add, which rounds
+   correctly for these x (P. Markstein, "Computation of elementary functions
+   on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990,
+   theorem 8.3).  No branch: independent reciprocals interleave. */
+__device__ __forceinline__ double rcp_normal(double x)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = __fma_rn(__fma_rn(-x, r, 1.0), r, r);
+    r = __fma_rn(__fma_rn(-x, r, 1.0), r, r);
+    r = __fma_rn(__fma_rn(-x, r, 1.0), r, r);
+    return r;
+}
+/* nonzero for the x that rcp_normal does not cover (or might not) */
+__device__ __forceinline__ unsigned rcp_odd(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    return (hi - (23u << 20) >= (2000u << 20)) | (lo == 0xffffffffu);
+}
+
 template <int G>
 __device__ __forceinline__ double group_max(double v)
 {
@@ -408,9 +430,26 @@ struct Cell {
         return group_max<G>(msk ? div_n(s) : -HUGE_VAL);
     }
 
-    /* CalcErrorWeightInvSquared (src/odevec.F90:706-716) */
+    /* CalcErrorWeightInvSquared (src/odevec.F90:706-716).  Up to 16 species
+       the reciprocals run without branches, side by side (a correctly rounded
+       __drcp_rn is a branch each, so twelve ran one after another): PRIMORDIAL
+       with FP32 factors 107.4 -> 102.9 ms, FP64 149.8 -> 144.5 ms
+       (1,048,576 cells).  Above, the second copy of the code costs more than
+       the chains (64 species: 474 against 498 ms). */
     __device__ __forceinline__ void weights(double rtol, double atol)
     {
+        if constexpr (ND <= 16) {
+            unsigned odd = 0;
+#pragma unroll
+            for (int j = 0; j < ND; ++j) {
+                const double x = rtol * fabs(y[Net::dyn(j)]) + atol;
+                odd |= rcp_odd(x);
+                const double w = rcp_normal(x);
+                w2[j] = w * w;
+            }
+            if (!odd)
+                return;
+        }
 #pragma unroll
         for (int j = 0; j < ND; ++j) {
             /* correctly rounded reciprocal: the same bits as 1.0 / x */
