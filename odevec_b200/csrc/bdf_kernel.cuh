@@ -1061,7 +1061,7 @@ __device__ __forceinline__ void bdf_run(const LaunchArgs& A)
     }
     alignas(16) double rates_local[C::NR];
     c.rT = rates_local;
-    int ph = PH_IDLE;
+    int ph = G == 1 && A.lanes > 0 && lane >= A.lanes ? PH_EXHAUSTED : PH_IDLE;
     int64_t cell = -1;
     bool write_y = false;
     __shared__ SoftSync soft;
@@ -1577,15 +1577,20 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
     kern<<<start, Cfg::BS, smem, stream>>>(P);
     return cudaGetLastError();
 }
+/* warps per SM of a launch of few cells: one per scheduler */
+constexpr int SPREAD_WARPS = 4;
+
 template <class Net, int G, class LUT, int STAGE>
 cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream)
 {
     using Cfg = StageCfg<STAGE>;
     auto kern = bdf_kernel<Net, G, LUT, STAGE>;
     constexpr size_t smem = Staging<Net, LUT, Cfg::SHM, Cfg::BS>::smem_bytes;
+    const bool chosen = block > 0 || grid > 0; /* the caller fixes the shape */
     if (Cfg::SHM || block <= 0 || block > Cfg::BS)
         block = Cfg::BS;
     static int cached_grid[2] = {0, 0};
+    static int cached_sms = 0;
     if (cached_grid[0] == 0 || cached_grid[1] != block) {
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
@@ -1598,8 +1603,36 @@ cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem);
         cached_grid[0] = sms * (per_sm > 0 ? per_sm : 1);
         cached_grid[1] = block;
+        cached_sms = sms;
     }
-    if (grid <= 0) {
+    LaunchArgs b = a;
+    if (Net::ND <= 32 && !chosen && a.ncells <= (int64_t)cached_sms * SPREAD_WARPS * 32) {
+        /* Few cells: over all SMs, at most one warp per scheduler and only as
+           many lanes per warp as that takes.  The time is that of the longest
+           cells' chain of steps then, and a warp's trip is the shorter the
+           fewer cells share it and the fewer warps share its scheduler.
+           PRIMORDIAL with FP32 factors, in blocks of 256 cells one after the
+           other / four warps per SM / eight warps per SM: 1,000 cells 8.4 /
+           4.6 / 5.4 ms, 4,096 cells 8.9 / 6.1 / 6.7, 8,192 cells 8.7 / 6.4 /
+           7.7, 16,384 cells 9.2 / 7.5 / 8.4; from 32,768 cells on full warps
+           are as fast or faster (9.4 against 9.8).  Not for large networks,
+           whose warps live from sharing instruction fetches (SYN64 FP64, 3,001
+           cells: 186 ms spread, 168 ms in 256-cell blocks). */
+        int64_t groups, lanes = 1; /* work items: cells, or lockstep groups (a warp each) */
+        groups = G == 1 ? a.ncells : (a.ncells + 31) / 32;
+        int64_t warps = (groups + cached_sms - 1) / cached_sms; /* per SM */
+        const int64_t most = Cfg::BS / 32 < SPREAD_WARPS ? Cfg::BS / 32 : SPREAD_WARPS;
+        if (warps > most)
+            warps = most;
+        if (G == 1)
+            lanes = (groups + cached_sms * warps - 1) / (cached_sms * warps);
+        b.lanes = (int32_t)(lanes < 32 ? lanes : 32);
+        block = (int)(32 * warps);
+        const int64_t per_block = warps * (G == 1 ? (int64_t)b.lanes : 1);
+        grid = (int)((groups + per_block - 1) / per_block);
+        if (grid < 1)
+            grid = 1;
+    } else if (grid <= 0) {
         grid = cached_grid[0];
         const int64_t warps_needed = (a.ncells + 31) / 32;
         const int64_t blocks_needed = (warps_needed * 32 + block - 1) / block;
@@ -1608,7 +1641,7 @@ cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream
         if (grid < 1)
             grid = 1;
     }
-    kern<<<grid, block, smem, stream>>>(a);
+    kern<<<grid, block, smem, stream>>>(b);
     return cudaGetLastError();
 }
 

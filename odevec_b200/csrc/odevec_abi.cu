@@ -611,6 +611,7 @@ static int32_t solve_impl(odevec_solver* s, int64_t ncells, int64_t stride, doub
     a.yield = s->yield;
     a.order = nullptr;
     a.rates = cont ? s->rate_cur : nullptr;
+    a.lanes = 0;
     cudaStream_t st = (cudaStream_t)stream;
     /* a continuation keeps the work counter (and the failure count) of the
        solve it continues */
@@ -1036,6 +1037,7 @@ extern "C" int32_t odevec_solve_noalloc(const char* network, const odevec_opts* 
     a.yield = nullptr;
     a.order = nullptr;
     a.rates = nullptr;
+    a.lanes = 0;
     const NetEntry& e = g_nets[ni];
     const int lu = o.precision == OV_PREC_FP32_LU ? 1 : 0;
     ov::launch_fn fn = o.precision == OV_PREC_FP64 ? e.exact : e.fma;

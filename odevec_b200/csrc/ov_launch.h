@@ -64,6 +64,9 @@ struct LaunchArgs {
        (STAGE_RATES) earlier on the stream; null: each cell evaluates its
        own as it is set up */
     double* rates;
+    /* per-cell control: lanes of each warp that take cells (1..32; 0: all),
+       chosen by the launcher */
+    int32_t lanes;
 };
 
 /* "staging" that fills LaunchArgs::rates instead of solving */

@@ -46,3 +46,28 @@ def test_rate_table_sizes(gpu_lib, oracle):
             _same(_gpu(gpu_lib, ode, wls[n]), _oracle(oracle, wls[n]))
     finally:
         gpu_lib.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("n", [1, 31, 148, 149, 593, 18944, 18945])
+def test_few_cells_shapes(gpu_lib, oracle, n):
+    """Launches of few cells: one lane of one warp, one warp per SM, a second
+    warp on an SM, several lanes per warp, the last size of the rule and the
+    first beyond it."""
+    wl = W.orego(ncells=n, seed=3)
+    wl.t_stop *= 0.05
+    ode = _solver(gpu_lib, wl)
+    try:
+        _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl))
+    finally:
+        gpu_lib.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("groups", [1, 148, 149, 592, 593])
+def test_few_groups_shapes(gpu_lib, oracle, groups):
+    """The same for lockstep groups of 32 cells, a warp each."""
+    wl = W.rober(ncells=32 * groups, seed=5)
+    ode = _solver(gpu_lib, wl)
+    try:
+        _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl))
+    finally:
+        gpu_lib.CloseOdevec(ode)
