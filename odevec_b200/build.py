@@ -6,7 +6,8 @@ parallel:
 * mode ``exact``: ``--fmad=false`` - no fused multiply-add, so every product
   and sum is rounded separately exactly as in the CPU oracle (G = 1 and 32,
   FP64 LU);
-* mode ``fma``: ``--fmad=true`` (G = 1 and 32; FP64 LU and FP32 LU).
+* mode ``fma``: ``--fmad=true`` (G = 1 and 32; FP64 LU and FP32 LU; OV_FUSED
+  is defined).
 
 The kernel template is instantiated in a namespace named after the mode, so
 the two modes never share a symbol.  The C-ABI layer (csrc/odevec_abi.cu) is
@@ -32,7 +33,7 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
                  "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
-MODES = {"exact": ["--fmad=false"], "fma": ["--fmad=true"]}
+MODES = {"exact": ["--fmad=false"], "fma": ["--fmad=true", "-DOV_FUSED=1"]}
 
 
 def variants():

@@ -172,6 +172,72 @@ __device__ __forceinline__ bool group_any(bool b)
     return b;
 }
 
+/* The choice of CalcStepSizeOrder (src/odevec.F90:547-618) from the squared
+   norms of the three candidates (x_down read only with has_down, x_up only
+   with has_up): returns the step-size factor; loc = 1, 2, 3 for order - 1,
+   the same order and order + 1, big when the factor reaches 1.1, so that the
+   order changes.  The literals 1.3, 1.2, 1.4 and 1.1 are single precision in
+   the reference.
+
+   Of the three candidate factors only one is used: the largest if it reaches
+   1.1, else the one of the same order.  Which one that is follows from
+   single-precision estimates (relative error below 1e-4) unless two
+   candidates, or the largest and 1.1, lie within 1e-3 of each other; then all
+   are evaluated.  So a lane evaluates one root, quotient and power instead of
+   three, each kept value the same IEEE expression as in the reference.  Bound
+   by the chain of dependent FP64 operations of a power (1,048,576 PRIMORDIAL
+   cells with FP32 factors: 109.3 -> 107.4 ms; a lockstep group evaluated three
+   powers one after another). */
+__device__ __forceinline__ double step_choice(int order, bool has_down, bool has_up, double x_down, double x_same,
+                                              double x_up, int& loc_out, bool& big_out)
+{
+    /* candidate loc = 1, 2, 3: 1 / (c * (norm / tau)^(1/k) + 1e-6) */
+    auto factor = [&](int loc) {
+        const double x = loc == 1 ? x_down : (loc == 2 ? x_same : x_up);
+        const double cc = loc == 1 ? (double)1.3f : (loc == 2 ? (double)1.2f : (double)1.4f);
+        const double n = (x < 0.0 ? x : sqrt(x)) / c_tau[order][loc - 1];
+        return 1.0 / (cc * ov_pow_sel(n, c_inv[order + loc - 1]) + 1e-6);
+    };
+    auto estimate = [&](double x, float cc, int loc) {
+        const int hi = __double2hiint(x);
+        const float m = __int_as_float(0x3f800000 | ((hi & 0xfffff) << 3));
+        const float l = (float)((hi >> 20) - 1023) + __log2f(m);
+        return cc * exp2f((0.5f * l - __log2f((float)c_tau[order][loc - 1])) * (float)c_inv[order + loc - 1])
+               + 1e-6f;
+    };
+    const float e_same = estimate(x_same, 1.2f, 2);
+    const float e_down = has_down ? estimate(x_down, 1.3f, 1) : HUGE_VALF;
+    const float e_up = has_up ? estimate(x_up, 1.4f, 3) : HUGE_VALF;
+    const float best = fminf(e_same, fminf(e_down, e_up));
+    const float near_best = best * 1.001f;
+    const bool one_best = (e_same <= near_best) + (e_down <= near_best) + (e_up <= near_best) == 1;
+    const bool below = best * 1.1f > 1.001f; /* the largest factor is below 1.1 */
+    const bool above = best * 1.1f < 0.999f;
+    /* infinities and NaN (a negative squared norm) take the full comparison */
+    const bool finite = x_same >= 0.0 && x_same < HUGE_VAL && (!has_down || (x_down >= 0.0 && x_down < HUGE_VAL))
+                        && (!has_up || (x_up >= 0.0 && x_up < HUGE_VAL));
+    const bool clear = finite && (below || (above && one_best));
+    int loc = 2;
+    if (clear && above)
+        loc = e_down <= near_best ? 1 : (e_up <= near_best ? 3 : 2);
+    double s = factor(loc);
+    bool big = above;
+    if (!clear) {
+        const double same = s;
+        const double down = has_down ? factor(1) : 0.0;
+        const double up = has_up ? factor(3) : 0.0;
+        loc = 1;
+        double mx = down;
+        if (same > mx) { mx = same; loc = 2; }
+        if (up > mx) { mx = up; loc = 3; }
+        big = mx >= (double)1.1f;
+        s = big ? mx : same;
+    }
+    loc_out = loc;
+    big_out = big;
+    return s;
+}
+
 /* Shared-memory staging: per-lane arrays laid out [entry][lane] with a
    stride of the block size, so a warp's 32 lanes touch 32 consecutive
    words (no bank conflicts). */
@@ -237,7 +303,8 @@ template <> struct StageCfg<16> { static constexpr int SHM = 0; static constexpr
    whose lanes then wait longer for new cells) */
 template <> struct StageCfg<17> { static constexpr int SHM = 2; static constexpr bool SOFT = true;  static constexpr int BS = 384, MINB = 1, REFILL = 32, PERIOD = 4; };
 /* as 15 and 8 (soft lockstep, 256 or 384 threads) with the state vector y
-   in shared memory (networks above 32 solver species) */
+   in shared memory (networks above 32 solver species; where blk_kernel.cuh
+   covers the network, staging 18 is its kernel) */
 template <> struct StageCfg<18> { static constexpr int SHM = 4; static constexpr bool SOFT = true;  static constexpr int BS = 256, MINB = 1, REFILL = 16, PERIOD = 4; };
 template <> struct StageCfg<19> { static constexpr int SHM = 4; static constexpr bool SOFT = true;  static constexpr int BS = 384, MINB = 1, REFILL = 16, PERIOD = 4; };
 /* staging 3's shape (three 128-thread blocks per SM, so that blocks of
@@ -552,19 +619,7 @@ struct Cell {
         }
     }
 
-    /* CalcStepSizeOrder (src/odevec.F90:547-618); returns dt_scale.  The
-       literals 1.3, 1.2, 1.4 and 1.1 are single precision in the reference.
-
-       Of the three candidate factors (order - 1, same, + 1) only one is used:
-       the largest if it reaches 1.1, else the one of the same order.  Which
-       one that is follows from single-precision estimates (relative error
-       below 1e-4) unless two candidates, or the largest and 1.1, lie within
-       1e-3 of each other; then all are evaluated.  So a lane evaluates one
-       root, quotient and power instead of three, each kept value the same
-       IEEE expression as in the reference.  Bound by the chain of dependent
-       FP64 operations of a power (1,048,576 PRIMORDIAL cells with FP32
-       factors: 109.3 -> 107.4 ms; a lockstep group evaluated three powers one
-       after another). */
+    /* CalcStepSizeOrder (src/odevec.F90:547-618); returns dt_scale */
     __device__ __forceinline__ double step_size_order()
     {
         const int order = q;
@@ -580,48 +635,9 @@ struct Cell {
                 d[j] = en[j] - eno[j];
             x_up = wnorm_sq(d);
         }
-        /* candidate loc = 1, 2, 3: 1 / (c * (norm / tau)^(1/k) + 1e-6) */
-        auto factor = [&](int loc) {
-            const double x = loc == 1 ? x_down : (loc == 2 ? x_same : x_up);
-            const double cc = loc == 1 ? (double)1.3f : (loc == 2 ? (double)1.2f : (double)1.4f);
-            const double n = (x < 0.0 ? x : sqrt(x)) / c_tau[order][loc - 1];
-            return 1.0 / (cc * ov_pow_sel(n, c_inv[order + loc - 1]) + 1e-6);
-        };
-        auto estimate = [&](double x, float cc, int loc) {
-            const int hi = __double2hiint(x);
-            const float m = __int_as_float(0x3f800000 | ((hi & 0xfffff) << 3));
-            const float l = (float)((hi >> 20) - 1023) + __log2f(m);
-            return cc * exp2f((0.5f * l - __log2f((float)c_tau[order][loc - 1])) * (float)c_inv[order + loc - 1])
-                   + 1e-6f;
-        };
-        const float e_same = estimate(x_same, 1.2f, 2);
-        const float e_down = has_down ? estimate(x_down, 1.3f, 1) : HUGE_VALF;
-        const float e_up = has_up ? estimate(x_up, 1.4f, 3) : HUGE_VALF;
-        const float best = fminf(e_same, fminf(e_down, e_up));
-        const float near_best = best * 1.001f;
-        const bool one_best = (e_same <= near_best) + (e_down <= near_best) + (e_up <= near_best) == 1;
-        const bool below = best * 1.1f > 1.001f; /* the largest factor is below 1.1 */
-        const bool above = best * 1.1f < 0.999f;
-        /* infinities and NaN (a negative squared norm) take the full comparison */
-        const bool finite = x_same >= 0.0 && x_same < HUGE_VAL && (!has_down || (x_down >= 0.0 && x_down < HUGE_VAL))
-                            && (!has_up || (x_up >= 0.0 && x_up < HUGE_VAL));
-        const bool clear = finite && (below || (above && one_best));
-        int loc = 2;
-        if (clear && above)
-            loc = e_down <= near_best ? 1 : (e_up <= near_best ? 3 : 2);
-        double s = factor(loc);
-        bool big = above;
-        if (!clear) {
-            const double same = s;
-            const double down = has_down ? factor(1) : 0.0;
-            const double up = has_up ? factor(3) : 0.0;
-            loc = 1;
-            double mx = down;
-            if (same > mx) { mx = same; loc = 2; }
-            if (up > mx) { mx = up; loc = 3; }
-            big = mx >= (double)1.1f;
-            s = big ? mx : same;
-        }
+        int loc;
+        bool big;
+        double s = step_choice(order, has_down, has_up, x_down, x_same, x_up, loc, big);
         if (big) {
             if (loc == 1) {
                 if (order != 1)
@@ -1685,6 +1701,7 @@ constexpr bool hist_fits_max()
 }  // namespace OV_MODE_NS
 }  // namespace ov
 
+#include "blk_kernel.cuh"
 #include "wpc_kernel.cuh"
 
 /* Defines the launcher of one network variant in the current mode.
@@ -1700,7 +1717,8 @@ constexpr bool hist_fits_max()
    of 256 or 512 (networks above 32 solver species); 17 = as 12 refilling on
    every 32nd trip; 18, 19 = as 8 in one block of 256 or 384 with the state
    vector in shared memory, 20 = as 3 with the state vector in shared memory
-   (18-20: networks above 32 solver species); 21 = as 3 with the history in
+   (18-20: networks above 32 solver species; 18 is the block-per-32-cells
+   kernel of blk_kernel.cuh for the networks that it covers); 21 = as 3 with the history in
    shared memory and the block in soft lockstep (up to 12 solver species).  With per-cell control stagings 2-6 and 8-16 refill idle
    lanes on every 16th trip, 17 on every 32nd, staging 1 on every trip.
    Stages 2-21 exist for per-cell control (G = 1). */
@@ -1745,7 +1763,10 @@ constexpr bool hist_fits_max()
             if constexpr (NET::ND > 32) {                                                    \
                 OV_STAGE_CASE(NET, double, 15)                                               \
                 OV_STAGE_CASE(NET, double, 16)                                               \
-                if constexpr (y_fits<NET, 256>()) {                                          \
+                if constexpr (blk_ok<NET, double>()) {                                       \
+                    if (stage == 18)                                                         \
+                        return launch_blk<NET, double>(a, grid, s);                          \
+                } else if constexpr (y_fits<NET, 256>()) {                                   \
                     OV_STAGE_CASE(NET, double, 18)                                           \
                 }                                                                            \
                 if constexpr (y_fits<NET, 128>()) {                                          \
@@ -1798,7 +1819,10 @@ constexpr bool hist_fits_max()
                 if constexpr (NET::ND > 32) {                                                \
                     OV_STAGE_CASE(NET, float, 15)                                            \
                     OV_STAGE_CASE(NET, float, 16)                                            \
-                    if constexpr (y_fits<NET, 256>()) {                                      \
+                    if constexpr (blk_ok<NET, float>()) {                                    \
+                        if (stage == 18)                                                     \
+                            return launch_blk<NET, float>(a, grid, s);                       \
+                    } else if constexpr (y_fits<NET, 256>()) {                               \
                         OV_STAGE_CASE(NET, float, 18)                                        \
                     }                                                                        \
                     if constexpr (y_fits<NET, 128>()) {                                      \

@@ -291,6 +291,20 @@ OV_HD static OV_INLINE double ov_pow_sel(double x, double y)
     return v;
 }
 
+#ifdef __cplusplus
+/* the same between the statements of a factorisation or solve on an LU of
+   accessor type A: left out where a kernel's accessor says so */
+template <class A>
+struct ov_lu_fenced {
+    static constexpr bool value = true;
+};
+#define OV_SCHED_LU(A)                       \
+    do {                                     \
+        if constexpr (ov_lu_fenced<A>::value) \
+            OV_SCHED();                      \
+    } while (0)
+#endif
+
 /* Pivots of the numeric LU.  In FP64 the factorisation and the solves divide
    by each pivot as the reference does (src/odevec.F90:906-969, :864-889).
    An FP32 LU stores each pivot's reciprocal in place once the pivot is final

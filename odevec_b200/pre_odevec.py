@@ -736,14 +736,14 @@ SCHED_EVERY = 16
 SCHED_EVERY_RHS = 4
 
 
-def _fenced(lines: List[str], every: int, on: bool, indent: str = "    ") -> List[str]:
+def _fenced(lines: List[str], every: int, on: bool, indent: str = "    ", fence: str = "OV_SCHED();") -> List[str]:
     if not on:
         return lines
     out = []
     for k, ln in enumerate(lines):
         out.append(ln)
         if (k + 1) % every == 0 and k + 1 < len(lines):
-            out.append(indent + "OV_SCHED();")
+            out.append(indent + fence)
     return out
 
 
@@ -861,7 +861,7 @@ def emit_cuda_header(sysm: System) -> str:
                                          [_remap_a(l, kmap) for l in _lu_solve_lines(sysm, dpos=dpos)])
     L.append("  template <class T, class A> OV_HD static OV_INLINE void lu_factor(A a) {")
     L.append("    (void)a;")
-    L += _fenced(["    " + ln for ln in f_lines], SCHED_EVERY, nd >= SCHED_MIN_ND)
+    L += _fenced(["    " + ln for ln in f_lines], SCHED_EVERY, nd >= SCHED_MIN_ND, fence="OV_SCHED_LU(A);")
     L.append("  }")
     L.append("  /* x = P^-1 r on the dynamic block; r, x over solver-state indices.  sc/isc")
     L.append("     scale entry i by sc[i] on the way in and isc[i] on the way out (pass")
@@ -871,7 +871,7 @@ def emit_cuda_header(sysm: System) -> str:
              "const double* OV_RESTRICT isc) {")
     L.append("#define OV_SC(i) (sc ? sc[i] : 1.0)")
     L.append("#define OV_ISC(i) (isc ? isc[i] : 1.0)")
-    L += _fenced(["    " + ln for ln in s_lines], SCHED_EVERY, nd >= SCHED_MIN_ND)
+    L += _fenced(["    " + ln for ln in s_lines], SCHED_EVERY, nd >= SCHED_MIN_ND, fence="OV_SCHED_LU(A);")
     L.append("#undef OV_SC")
     L.append("#undef OV_ISC")
     L.append("  }")

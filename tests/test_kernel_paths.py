@@ -71,3 +71,48 @@ def test_few_groups_shapes(gpu_lib, oracle, groups):
         _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl))
     finally:
         gpu_lib.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("n,mask,neg", [(1, False, False), (33, True, False), (149, False, True), (4737, True, True)])
+def test_block_kernel(gpu_lib, oracle, n, mask, neg):
+    """A large network, eight warps per 32 cells: one cell, a second block,
+    more cells than SMs, more than all blocks hold; masked cells and
+    CheckNegatives; then a continuation from the kept state."""
+    import torch
+    S = gpu_lib
+    wl = W.syn64(ncells=n, seed=4)
+    wl.t_stop[:] = 10.0 ** np.random.default_rng(2).uniform(-3.0, 3.0, n)
+    m = None
+    if mask:
+        m = np.random.default_rng(1).random(n) > 0.2
+        m[0] = True
+    ode = _solver(S, wl, CheckNegatives=neg, staging=18)
+    try:
+        y = torch.tensor(wl.y, device="cuda")
+        ws = S.Workspace(ode, n)
+        ows = oracle.workspace(wl.network, n)
+        oy, ot, od = wl.y, wl.t0, wl.dt0
+        t, d = torch.tensor(wl.t0, device="cuda"), torch.tensor(wl.dt0, device="cuda")
+        for k, resume in enumerate((False, True, "en_old")):
+            ts = wl.t_stop * 2.0 ** k
+            t, d = S.SolveODE(ode, t, d, torch.tensor(ts, device="cuda"), y, Mask=m, workspace=ws, resume=resume)
+            torch.cuda.synchronize()
+            oy, ot, od, ost, ostats = oracle.solve(wl.network, oy, ot, od, ts, wl.rtol, wl.atol, wl.dt_min, group=1,
+                                                   mask=m, check_negatives=neg, ws=ows, resume=resume)
+            _same([a.cpu().numpy() for a in (y, t, d, ode.status, ode.stats)], (oy, ot, od, ost, ostats))
+    finally:
+        S.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("precision", ["fp64_fma", "fp32_lu"])
+def test_block_kernel_forms(gpu_lib, precision):
+    """The contracted forms give the bits of a thread per cell (staging 15)."""
+    wl = W.syn64(ncells=300, seed=9)
+    got = []
+    for staging in (18, 15):
+        ode = _solver(gpu_lib, wl, precision=precision, staging=staging, escalation=False)
+        try:
+            got.append(_gpu(gpu_lib, ode, wl))
+        finally:
+            gpu_lib.CloseOdevec(ode)
+    _same(got[0], got[1])
