@@ -1504,95 +1504,6 @@ __global__ void __launch_bounds__(StageCfg<STAGE>::BS, StageCfg<STAGE>::MINB)
     bdf_run<Net, G, LUT, STAGE>(A);
 }
 
-/* ---- several networks in one launch ---------------------------------- */
-/* one 384-thread block per SM in soft lockstep, each thread's state vector
-   in shared memory (rows sized for the largest network of the set): the
-   register budget of staging 3, without the instruction-fetch stalls of a
-   large network's code, and with the large network's state reloaded from
-   shared memory instead of spilled (SYN64: 1.49x over staging 1); every
-   warp of a block runs the same job at a time, so the lockstep keeps them
-   on the same code */
-constexpr int MULTI_STAGE = 19;
-
-template <class LUT, class... Nets>
-constexpr size_t multi_smem_bytes()
-{
-    size_t m = 0;
-    ((m = Staging<Nets, LUT, StageCfg<MULTI_STAGE>::SHM, StageCfg<MULTI_STAGE>::BS>::smem_bytes > m
-              ? Staging<Nets, LUT, StageCfg<MULTI_STAGE>::SHM, StageCfg<MULTI_STAGE>::BS>::smem_bytes
-              : m),
-     ...);
-    return m;
-}
-
-template <class LUT, class... Nets>
-struct MultiDispatch {
-    __device__ __forceinline__ static void run(int, const LaunchArgs&) {}
-};
-template <class LUT, class Net0, class... Rest>
-struct MultiDispatch<LUT, Net0, Rest...> {
-    __device__ __forceinline__ static void run(int idx, const LaunchArgs& A)
-    {
-        if (idx == 0)
-            bdf_run<Net0, 1, LUT, MULTI_STAGE>(A);
-        else
-            MultiDispatch<LUT, Rest...>::run(idx - 1, A);
-    }
-};
-
-template <class LUT, class... Nets>
-__global__ void __launch_bounds__(StageCfg<MULTI_STAGE>::BS, StageCfg<MULTI_STAGE>::MINB)
-    bdf_multi_kernel(const __grid_constant__ MultiArgs P)
-{
-    int first = 0;
-    while (first + 1 < P.njobs && (int)blockIdx.x >= P.block_start[first + 1])
-        ++first;
-    for (int k = 0; k < P.njobs; ++k) {
-        const int j = (first + k) % P.njobs;
-        MultiDispatch<LUT, Nets...>::run(P.net[j], P.job[j]);
-    }
-}
-
-/* Launches the multi-network kernel on P (block ranges filled in here in
-   proportion to the jobs' cells, at least one block per job). */
-template <class LUT, class... Nets>
-cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
-{
-    using Cfg = StageCfg<MULTI_STAGE>;
-    auto kern = bdf_multi_kernel<LUT, Nets...>;
-    constexpr size_t smem = multi_smem_bytes<LUT, Nets...>();
-    static_assert(smem <= 226 * 1024, "the set's largest state vectors exceed a block's shared memory");
-    static int cached_grid = 0;
-    if (cached_grid == 0) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess)
-                return e;
-        }
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Cfg::BS, smem);
-        cached_grid = sms * (per_sm > 0 ? per_sm : 1);
-    }
-    int64_t total = 0;
-    for (int j = 0; j < P.njobs; ++j)
-        total += P.job[j].ncells;
-    int grid = cached_grid;
-    if (grid < P.njobs)
-        grid = P.njobs;
-    int start = 0;
-    for (int j = 0; j < P.njobs; ++j) {
-        P.block_start[j] = start;
-        int nb = total > 0 ? (int)((double)grid * (double)P.job[j].ncells / (double)total) : 0;
-        if (nb < 1)
-            nb = 1;
-        start += nb;
-    }
-    P.block_start[P.njobs] = start;
-    kern<<<start, Cfg::BS, smem, stream>>>(P);
-    return cudaGetLastError();
-}
 /* warps per SM of a launch of few cells: one per scheduler */
 constexpr int SPREAD_WARPS = 4;
 
@@ -1703,6 +1614,124 @@ constexpr bool hist_fits_max()
 
 #include "blk_kernel.cuh"
 #include "wpc_kernel.cuh"
+
+namespace ov {
+namespace OV_MODE_NS {
+
+/* ---- several networks in one launch ---------------------------------- */
+/* One block of 256 threads per SM with all the registers of a thread.  A job
+   runs as its network runs best alone: a large network as one block per 32
+   cells (blk_kernel.cuh), another as staging 9 (soft lockstep, the history in
+   shared memory) or, where a history does not fit, staging 15.  The blocks are
+   shared out in proportion to cells times LU entries, an estimate of the
+   jobs' work; a block whose job has no cells left takes cells of the others.
+   16,384 ROBER, 65,536 PRIMORDIAL and 4,096 SYN64 cells, FP32-LU: 190 ms with
+   every network on one 384-thread block per SM and shares by cells alone,
+   46 ms so. */
+template <class Net, class LUT>
+struct MultiJob {
+    static constexpr int STAGE = hist_fits<Net, 256>() ? 9 : 15;
+    static constexpr bool BLOCK = blk_ok<Net, LUT>();
+    static constexpr size_t smem()
+    {
+        if constexpr (BLOCK)
+            return BlkLayout<Net, LUT>::smem_bytes;
+        else
+            return Staging<Net, LUT, StageCfg<STAGE>::SHM, StageCfg<STAGE>::BS>::smem_bytes;
+    }
+    __device__ __forceinline__ static void run(const LaunchArgs& A)
+    {
+        /* both begin with a barrier, so no warp touches the shared memory of
+           this job while another still works on the one before */
+        if constexpr (BLOCK)
+            blk_run<Net, LUT>(A);
+        else
+            bdf_run<Net, 1, LUT, STAGE>(A);
+    }
+};
+constexpr int MULTI_BS = 256;
+static_assert(32 * BLK_WARPS == MULTI_BS && StageCfg<9>::BS == MULTI_BS && StageCfg<15>::BS == MULTI_BS &&
+                  StageCfg<9>::SOFT && StageCfg<15>::SOFT,
+              "the jobs of a multi-network launch share one block shape and start with a barrier");
+
+template <class LUT, class... Nets>
+constexpr size_t multi_smem_bytes()
+{
+    size_t m = 0;
+    ((m = MultiJob<Nets, LUT>::smem() > m ? MultiJob<Nets, LUT>::smem() : m), ...);
+    return m;
+}
+
+template <class LUT, class... Nets>
+struct MultiDispatch {
+    __device__ __forceinline__ static void run(int, const LaunchArgs&) {}
+};
+template <class LUT, class Net0, class... Rest>
+struct MultiDispatch<LUT, Net0, Rest...> {
+    __device__ __forceinline__ static void run(int idx, const LaunchArgs& A)
+    {
+        if (idx == 0)
+            MultiJob<Net0, LUT>::run(A);
+        else
+            MultiDispatch<LUT, Rest...>::run(idx - 1, A);
+    }
+};
+
+template <class LUT, class... Nets>
+__global__ void __launch_bounds__(MULTI_BS, 1) bdf_multi_kernel(const __grid_constant__ MultiArgs P)
+{
+    int first = 0;
+    while (first + 1 < P.njobs && (int)blockIdx.x >= P.block_start[first + 1])
+        ++first;
+    for (int k = 0; k < P.njobs; ++k) {
+        const int j = (first + k) % P.njobs;
+        MultiDispatch<LUT, Nets...>::run(P.net[j], P.job[j]);
+    }
+}
+
+/* Launches the multi-network kernel on P (block ranges filled in here in
+   proportion to the jobs' work, at least one block per job). */
+template <class LUT, class... Nets>
+cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
+{
+    auto kern = bdf_multi_kernel<LUT, Nets...>;
+    constexpr size_t smem = multi_smem_bytes<LUT, Nets...>();
+    static_assert(smem <= 226 * 1024, "the set's largest state vectors exceed a block's shared memory");
+    static int cached_grid = 0;
+    if (cached_grid == 0) {
+        int dev = 0, sms = 0, per_sm = 0;
+        cudaGetDevice(&dev);
+        if (smem > 48 * 1024) {
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess)
+                return e;
+        }
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MULTI_BS, smem);
+        cached_grid = sms * (per_sm > 0 ? per_sm : 1);
+    }
+    const int nnz[] = {Nets::NNZ...};
+    double total = 0.0;
+    for (int j = 0; j < P.njobs; ++j)
+        total += (double)P.job[j].ncells * nnz[P.net[j]];
+    int grid = cached_grid;
+    if (grid < P.njobs)
+        grid = P.njobs;
+    int start = 0;
+    for (int j = 0; j < P.njobs; ++j) {
+        P.block_start[j] = start;
+        int nb = total > 0.0 ? (int)(grid * ((double)P.job[j].ncells * nnz[P.net[j]]) / total) : 0;
+        if (nb < 1)
+            nb = 1;
+        start += nb;
+    }
+    P.block_start[P.njobs] = start;
+    kern<<<start, MULTI_BS, smem, stream>>>(P);
+    return cudaGetLastError();
+}
+
+}  // namespace OV_MODE_NS
+}  // namespace ov
 
 /* Defines the launcher of one network variant in the current mode.
    stage: 1 = thread-local arrays, 2 blocks of 128 per SM; 2 = history and

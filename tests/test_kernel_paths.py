@@ -116,3 +116,28 @@ def test_block_kernel_forms(gpu_lib, precision):
         finally:
             gpu_lib.CloseOdevec(ode)
     _same(got[0], got[1])
+
+
+@pytest.mark.parametrize("cells", [(32, 1, 1), (4096, 5000, 40), (33, 70, 700)])
+def test_multi_block_jobs(gpu_lib, oracle, cells):
+    """Several networks in one launch with blocks that go from one job's kernel
+    to another's in either order."""
+    import torch
+    from odevec_b200.multi import SolveMany
+    S = gpu_lib
+    wls = [W.rober(cells[0], seed=2), W.primordial(cells[1], seed=2), W.syn64(cells[2], seed=2)]
+    wls[2].t_stop[:] = 1e2
+    odes, jobs = [], []
+    for wl in wls:
+        ode = _solver(S, wl, nvector=1)
+        odes.append(ode)
+        jobs.append((ode, *[torch.tensor(a, device="cuda") for a in (wl.t0, wl.dt0, wl.t_stop, wl.y)]))
+    try:
+        status = SolveMany(jobs, fused=True).run()
+        torch.cuda.synchronize()
+        for wl, job, st in zip(wls, jobs, status):
+            o = _oracle(oracle, wl, group=1)
+            _same([a.cpu().numpy() for a in (job[4], job[1], job[2], st)], o[:4])
+    finally:
+        for ode in odes:
+            S.CloseOdevec(ode)
