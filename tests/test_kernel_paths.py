@@ -141,3 +141,22 @@ def test_multi_block_jobs(gpu_lib, oracle, cells):
     finally:
         for ode in odes:
             S.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("n,shift", [(1, 0), (2, 0), (511, 0), (512, 0), (514, 0), (514, 1), (1025, 1)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_convert_widths(gpu_lib, oracle, n, shift, in_place):
+    """Even and odd cell counts, arrays that do not start on 16 bytes, blocks
+    that end inside a pair, the output over the input."""
+    import torch
+    from odevec_b200 import driver as D
+    rng = np.random.default_rng(n)
+    x = 10.0 ** rng.uniform(-20.0, 0.0, (16, n))
+    rho = 10.0 ** rng.uniform(-26.0, -18.0, n)
+    buf = torch.zeros(16 * n + 1, dtype=torch.float64, device="cuda")
+    a = buf[shift:shift + 16 * n].view(16, n)
+    r = torch.tensor(rho, device="cuda")
+    for direction in (D.OV_X2N, D.OV_N2X):
+        a.copy_(torch.tensor(x))
+        out = D.convert("PRIMORDIAL_CSC_FF", a, r, direction, out=a if in_place else None)
+        assert np.array_equal(out.cpu().numpy(), oracle.convert("PRIMORDIAL_CSC_FF", x, rho, direction))
