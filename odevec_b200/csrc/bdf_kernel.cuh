@@ -157,9 +157,13 @@ __device__ __forceinline__ double group_max(double v)
 {
     v = max_operand(v);
     if (G == 32) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            v = fmax(v, __shfl_xor_sync(FULL, v, o));
+        /* v is -infinity or non-negative, so its words order as integers:
+           the largest upper word, then the largest lower word beside it.  Two
+           integer reductions instead of ten shuffles and five comparisons */
+        const int hi = __double2hiint(v);
+        const int top = __reduce_max_sync(FULL, hi);
+        const unsigned low = __reduce_max_sync(FULL, hi == top ? (unsigned)__double2loint(v) : 0u);
+        v = __hiloint2double(top, (int)low);
     }
     return v;
 }
@@ -370,6 +374,57 @@ __device__ __forceinline__ void soft_leave(SoftSync* s, int lane)
 }
 
 
+/* An FP64 LU with the correctly rounded reciprocals of its pivots beside it.
+   A division by a pivot is then five dependent fused multiply-adds without a
+   branch: the quotient from the reciprocal, corrected twice with its exact
+   residual, which rounds correctly (P. Markstein, IBM J. Res. Dev. 34, 1990).
+   Operands for which that is not certain (far exponents, infinities, NaN, an
+   all-ones significand) are recorded in bad, and the caller repeats the work
+   with IEEE divisions.  The generated factorisation and solves pick these
+   overloads of ov_pivot and ov_divp by the accessor's entry type. */
+struct PivotRef {
+    double* p;
+    double* r;
+    unsigned* bad;
+    __device__ __forceinline__ operator double() const { return *p; }
+    __device__ __forceinline__ void operator=(double v) const { *p = v; }
+};
+
+template <class Net, class A>
+struct PivotLU {
+    A a;       /* the packed factors */
+    double* r; /* [ND] reciprocals, by pivot number */
+    unsigned* bad;
+    __device__ __forceinline__ PivotRef operator[](int i) const
+    {
+        const int k = Net::pivot_number(i);
+        return PivotRef{&a[i], r + (k < 0 ? 0 : k), bad};
+    }
+};
+
+template <class T>
+__device__ __forceinline__ T ov_pivot(const PivotRef& p)
+{
+    const double v = p;
+    const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu, lo = (unsigned)__double2loint(v);
+    /* outside [2^-400, 2^400) or all ones below */
+    *p.bad |= (hi - (623u << 20) >= (800u << 20)) | (lo == 0xffffffffu);
+    *p.r = rcp_normal(v);
+    return v;
+}
+
+template <class T>
+__device__ __forceinline__ T ov_divp(T x, const PivotRef& p)
+{
+    const double d = p, r = *p.r;
+    const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu, lo = (unsigned)__double2loint(x);
+    /* outside [2^-500, 2^500) and not zero */
+    *p.bad |= (hi - (523u << 20) >= (1000u << 20)) & ((hi | lo) != 0u);
+    double q = x * r;
+    q = __fma_rn(__fma_rn(-q, d, x), r, q);
+    return __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+
 template <class Net, class LUT, int SHM, int BS>
 struct Staging;
 
@@ -414,6 +469,20 @@ struct Cell {
     static constexpr int NNZ = Net::NNZ;
     static constexpr int NR = Net::NREA > 0 ? Net::NREA : 1;
     static constexpr bool SCALED = sizeof(LUT) == 4;
+    /* a small network's thread-local history is indexed by constants only,
+       the columns beyond the order predicated off, so that it lives in
+       registers.  With this, the reductions by words in lockstep groups, the
+       exact quotient by the species count and PivotLU (below): ROBER, one
+       lockstep group 0.54 -> 0.44 ms, 128 groups 0.60 -> 0.48 ms; OREGO,
+       65,536 cells FP64 13.3 (staging 2) -> 12.4 ms (staging 3) */
+    static constexpr bool REGH = ND <= 4 && SHM == 0;
+    /* FP64 pivots with their reciprocals (PivotLU) for small networks, whose
+       trip is a chain of dependent operations.  12 species: 175 against 145
+       ms (PRIMORDIAL, 1,048,576 cells, FP64; the second copy of the code
+       spills); with the reciprocals in the solves alone 146.  Not where the
+       matrix keeps entries of the factorisation before, which must not be
+       repeated. */
+    static constexpr bool PIV = !SCALED && ND <= 4 && !Net::HC_FD;
 
     typename Staging<Net, LUT, SHM, BS>::Hist yns; /* Nordsieck history y_NS(0:5) */
     /* 16-byte aligned, so that neighbouring entries can move in one 128-bit
@@ -425,6 +494,7 @@ struct Cell {
        shared memory, which the network code reloads instead of spilling */
     alignas(16) std::conditional_t<SHM == 4, double*, double[N]> y;
     typename Staging<Net, LUT, SHM, BS>::LU a; /* packed LU of the iteration matrix */
+    double* rp;                                /* PIV: reciprocals of its pivots */
     /* temperature part of the rates: an array of its own, not a member.  The
        set-up call that fills it takes its address, and as a member it would
        keep this whole object (state, weights, corrections, every control
@@ -441,6 +511,7 @@ struct Cell {
     double fz_add; /* 0, or NaN when a frozen species has a non-finite error weight */
     int q, swu, lju, fet, fc, it, ss_mode, wait;
     bool ujac, nuo, first, msk, fz_neg;
+    bool ieee; /* PIV: these factors need IEEE divisions */
     int status, attempts, steps, ltef, convf, newt, jacs, ppass;
 
     /* x / N for the full species count: for a power of two N the product
@@ -448,10 +519,20 @@ struct Cell {
        the same exact value), without the division's instruction sequence */
     __device__ __forceinline__ static double div_n(double x)
     {
-        if constexpr ((N & (N - 1)) == 0)
+        if constexpr ((N & (N - 1)) == 0) {
             return x * (1.0 / N);
-        else
-            return x / N;
+        } else {
+            /* the quotient from the rounded reciprocal, corrected twice with
+               its exact residual: correctly rounded (Markstein, as above)
+               where nothing underflows or overflows */
+            const double r = 1.0 / N;
+            double v = x * r;
+            v = __fma_rn(__fma_rn(-(double)N, v, x), r, v);
+            v = __fma_rn(__fma_rn(-(double)N, v, x), r, v);
+            if (x != 0.0 && (unsigned)__double2hiint(x) - (123u << 20) >= (1900u << 20))
+                v = x / N;
+            return v;
+        }
     }
 
     /* WeightedNorm1 (src/odevec.F90:669-684) over the solver state; the
@@ -490,7 +571,15 @@ struct Cell {
         double s = 0.0;
 #pragma unroll
         for (int j = 0; j < ND; ++j) {
-            const double e = yns[col][j];
+            double e;
+            if constexpr (REGH) {
+                e = yns[1][j];
+#pragma unroll
+                for (int k = 2; k <= MAXQ; ++k)
+                    e = k == col ? yns[k][j] : e;
+            } else {
+                e = yns[col][j];
+            }
             s = s + e * e * w2[j];
         }
         s = s + fz_add;
@@ -596,12 +685,23 @@ struct Cell {
     __device__ __forceinline__ void set_step(double dt_scale)
     {
         double dtt = 1.0;
-#pragma unroll 1
-        for (int k = 1; k <= q; ++k) {
-            dtt = dt_scale * dtt;
+        if constexpr (REGH) {
 #pragma unroll
-            for (int j = 0; j < ND; ++j)
-                yns[k][j] = yns[k][j] * dtt;
+            for (int k = 1; k <= MAXQ; ++k) {
+                dtt = dt_scale * dtt;
+#pragma unroll
+                for (int j = 0; j < ND; ++j)
+                    if (k <= q)
+                        yns[k][j] = yns[k][j] * dtt;
+            }
+        } else {
+#pragma unroll 1
+            for (int k = 1; k <= q; ++k) {
+                dtt = dt_scale * dtt;
+#pragma unroll
+                for (int j = 0; j < ND; ++j)
+                    yns[k][j] = yns[k][j] * dtt;
+            }
         }
         h = h * dt_scale;
         jchg = jchg * dt_scale;
@@ -610,12 +710,23 @@ struct Cell {
     /* UpdateNordsieck (src/odevec.F90:747-765) */
     __device__ __forceinline__ void update_nordsieck()
     {
-#pragma unroll 1
-        for (int k = 0; k <= q; ++k) {
-            const double c = lcoef(q, k);
+        if constexpr (REGH) {
 #pragma unroll
-            for (int j = 0; j < ND; ++j)
-                yns[k][j] = yns[k][j] + en[j] * c;
+            for (int k = 0; k <= MAXQ; ++k) {
+                const double c = lcoef(q, k);
+#pragma unroll
+                for (int j = 0; j < ND; ++j)
+                    if (k <= q)
+                        yns[k][j] = yns[k][j] + en[j] * c;
+            }
+        } else {
+#pragma unroll 1
+            for (int k = 0; k <= q; ++k) {
+                const double c = lcoef(q, k);
+#pragma unroll
+                for (int j = 0; j < ND; ++j)
+                    yns[k][j] = yns[k][j] + en[j] * c;
+            }
         }
     }
 
@@ -648,8 +759,16 @@ struct Cell {
                 if (order != MAXQ) {
                     const double c = lcoef(order, order);
 #pragma unroll
-                    for (int j = 0; j < ND; ++j)
-                        yns[order + 1][j] = c * en[j] / (order + 1.0);
+                    for (int j = 0; j < ND; ++j) {
+                        const double v = c * en[j] / (order + 1.0);
+                        if constexpr (REGH) {
+#pragma unroll
+                            for (int k = 2; k <= MAXQ; ++k)
+                                yns[k][j] = k == order + 1 ? v : yns[k][j];
+                        } else {
+                            yns[order + 1][j] = v;
+                        }
+                    }
                     q = order + 1;
                 } else
                     status = OV_ERR_ORDER;
@@ -745,18 +864,34 @@ struct Cell {
                 isc[j] = ov_pow2i(-hexp);
             }
         }
-        if constexpr (Net::LU_METHOD == 3) {
-            fd_jacobian(sc, isc);
-        } else {
-            double k[NR];
-            Net::rates_k(y, rT, k);
-            if constexpr (!SCALED)
-                Net::template jac<LUT>(y, k, lcoef(q, 0), h, a);
-            else
-                Net::template jac_scaled<LUT>(y, k, lcoef(q, 0), h, a, sc, isc);
+        ieee = false;
+#pragma unroll 1
+        for (;;) {
+            if constexpr (Net::LU_METHOD == 3) {
+                fd_jacobian(sc, isc);
+            } else {
+                double k[NR];
+                Net::rates_k(y, rT, k);
+                if constexpr (!SCALED)
+                    Net::template jac<LUT>(y, k, lcoef(q, 0), h, a);
+                else
+                    Net::template jac_scaled<LUT>(y, k, lcoef(q, 0), h, a, sc, isc);
+            }
+            /* for LUmethod 2 jac() wrote the symbolic factors */
+            if constexpr (PIV) {
+                if (!ieee) {
+                    unsigned bad = 0u;
+                    Net::template lu_factor<LUT>(PivotLU<Net, decltype(a)>{a, rp, &bad});
+                    if (bad) {
+                        ieee = true; /* once more from the matrix */
+                        continue;
+                    }
+                    break;
+                }
+            }
+            Net::template lu_factor<LUT>(a);
+            break;
         }
-        /* empty for LUmethod 2: jac() wrote the symbolic factors */
-        Net::template lu_factor<LUT>(a);
     }
 
     /* CalcJac_dense (src/odevec.F90:469-506), the DRPEPJ difference
@@ -839,6 +974,11 @@ struct Cell {
                 isc[j] = ov_pow2i(-sce[j]);
             }
             Net::template lu_solve<LUT>(a, res, den, sc, isc);
+        } else if constexpr (PIV) {
+            unsigned bad = ieee ? 1u : 0u;
+            Net::template lu_solve<LUT>(PivotLU<Net, decltype(a)>{a, rp, &bad}, res, den, nullptr, nullptr);
+            if (bad)
+                Net::template lu_solve<LUT>(a, res, den, nullptr, nullptr);
         } else {
             Net::template lu_solve<LUT>(a, res, den, nullptr, nullptr);
         }
@@ -878,10 +1018,20 @@ struct Cell {
         const double rel_t = (tstop - t) / h;
 #pragma unroll
         for (int j = 0; j < ND; ++j) {
-            double acc = yns[q][j];
+            double acc;
+            if constexpr (REGH) {
+                acc = yns[MAXQ][j];
+#pragma unroll
+                for (int k = MAXQ - 1; k >= 0; --k) {
+                    const double next = yns[k][j] + rel_t * acc;
+                    acc = k < q ? next : yns[k][j];
+                }
+            } else {
+                acc = yns[q][j];
 #pragma unroll 1
-            for (int k = q - 1; k >= 0; --k)
-                acc = yns[k][j] + rel_t * acc;
+                for (int k = q - 1; k >= 0; --k)
+                    acc = yns[k][j] + rel_t * acc;
+            }
             if (msk)
                 y[Net::dyn(j)] = acc;
         }
@@ -914,7 +1064,7 @@ struct Cell {
     __device__ __forceinline__ void save_state(double* ws, int64_t n, int64_t cell) const
     {
         int f = 0;
-#pragma unroll 1
+#pragma unroll (REGH ? MAXQ + 1 : 1)
         for (int k = 0; k <= MAXQ; ++k)
 #pragma unroll
             for (int j = 0; j < ND; ++j)
@@ -936,7 +1086,7 @@ struct Cell {
     __device__ __forceinline__ void load_state(const double* ws, int64_t n, int64_t cell)
     {
         int f = 0;
-#pragma unroll 1
+#pragma unroll (REGH ? MAXQ + 1 : 1)
         for (int k = 0; k <= MAXQ; ++k)
 #pragma unroll
             for (int j = 0; j < ND; ++j)
@@ -1075,6 +1225,8 @@ __device__ __forceinline__ void bdf_run(const LaunchArgs& A)
         if constexpr (C::NNZ > 16 && (sizeof(LUT) == 8 || C::NNZ <= 128))
             asm volatile("" ::"l"(&lu_local[0]) : "memory");
     }
+    double rcp_local[C::PIV ? ND : 1];
+    c.rp = rcp_local;
     alignas(16) double rates_local[C::NR];
     c.rT = rates_local;
     int ph = G == 1 && A.lanes > 0 && lane >= A.lanes ? PH_EXHAUSTED : PH_IDLE;

@@ -51,6 +51,14 @@ struct ov_net_rober_dense_none_lu3 {
   }
   /* in-place numeric LU of the packed dynamic block a[0..NNZ-1]; A is a
      pointer or an accessor whose operator[] yields T& */
+  /* packed index of a pivot -> its number 0..ND-1; -1 for other entries */
+  OV_HD static constexpr int pivot_number(int i) {
+    constexpr int p[3] = {0, 4, 8};
+    for (int k = 0; k < 3; ++k)
+      if (p[k] == i)
+        return k;
+    return -1;
+  }
   template <class T, class A> OV_HD static OV_INLINE void lu_factor(A a) {
     (void)a;
     a[0] = ov_pivot<T>(a[0]);

@@ -859,6 +859,17 @@ def emit_cuda_header(sysm: System) -> str:
     L.append("     pointer or an accessor whose operator[] yields T& */")
     f_lines, s_lines = reciprocal_pivots(_reduce_lines(_lu_factor_lines(sysm), kmap),
                                          [_remap_a(l, kmap) for l in _lu_solve_lines(sysm, dpos=dpos)])
+    if nd <= 4:
+        # the kernel keeps reciprocals of a small network's FP64 pivots
+        piv = sorted(int(m.group(1)) for m in (re.match(r"a\[(\d+)\] = ov_pivot", ln) for ln in f_lines) if m)
+        L.append("  /* packed index of a pivot -> its number 0..ND-1; -1 for other entries */")
+        L.append("  OV_HD static constexpr int pivot_number(int i) {")
+        L.append("    constexpr int p[%d] = {%s};" % (len(piv), ", ".join("%d" % v for v in piv)))
+        L.append("    for (int k = 0; k < %d; ++k)" % len(piv))
+        L.append("      if (p[k] == i)")
+        L.append("        return k;")
+        L.append("    return -1;")
+        L.append("  }")
     L.append("  template <class T, class A> OV_HD static OV_INLINE void lu_factor(A a) {")
     L.append("    (void)a;")
     L += _fenced(["    " + ln for ln in f_lines], SCHED_EVERY, nd >= SCHED_MIN_ND, fence="OV_SCHED_LU(A);")

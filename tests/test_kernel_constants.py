@@ -66,3 +66,28 @@ def test_reciprocal_iteration(mantissa):
             for _ in range(3):
                 r = fma(fma(-x, r, 1.0), r, r)
             assert r == want
+
+
+@pytest.mark.parametrize("kind", ["pivot", "count"])
+def test_quotient_iteration(kind):
+    """The kernel's branch-free quotients -- by a pivot, and by a species count
+    that is no power of two -- are correctly rounded: the product with the
+    rounded reciprocal, corrected twice with its exact residual."""
+    import random
+    from fractions import Fraction as F
+    rng = random.Random(11)
+    fma = lambda a, b, c: float(F(a) * F(b) + F(c))
+    for _ in range(3000):
+        if kind == "pivot":
+            d = math.ldexp(1.0 + rng.choice([rng.getrandbits(52), rng.getrandbits(4), (1 << 52) - 2 - rng.getrandbits(4)])
+                           * 2.0 ** -52, rng.randint(-390, 390)) * rng.choice([-1.0, 1.0])
+            e = rng.randint(-490, 490)
+        else:
+            d, e = float(rng.choice([3, 5, 6, 7, 9, 12])), rng.randint(-890, 990)
+        x = math.ldexp(1.0 + rng.choice([rng.getrandbits(52), rng.getrandbits(4), (1 << 52) - 1 - rng.getrandbits(4)])
+                       * 2.0 ** -52, e)
+        r = 1.0 / d
+        q = x * r
+        q = fma(fma(-q, d, x), r, q)
+        q = fma(fma(-q, d, x), r, q)
+        assert q == x / d

@@ -160,3 +160,20 @@ def test_convert_widths(gpu_lib, oracle, n, shift, in_place):
         a.copy_(torch.tensor(x))
         out = D.convert("PRIMORDIAL_CSC_FF", a, r, direction, out=a if in_place else None)
         assert np.array_equal(out.cpu().numpy(), oracle.convert("PRIMORDIAL_CSC_FF", x, rho, direction))
+
+
+@pytest.mark.parametrize("group,scale", [(1, 1e-9), (1, 1e4), (32, 1.0)])
+def test_small_network_far_operands(gpu_lib, oracle, group, scale):
+    """Three species: states far below and above the usual range (zeros among
+    them), whose divisions leave or approach the range of the branch-free
+    quotients."""
+    wl = W.rober(ncells=96, seed=8)
+    wl.y *= scale
+    wl.y[:, ::5] *= 1e-290
+    wl.y[1, ::3] = 0.0
+    wl.t_stop[:] = 1e2
+    ode = _solver(gpu_lib, wl, nvector=group, max_attempts=3000)
+    try:
+        _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl, group=group, max_attempts=3000))
+    finally:
+        gpu_lib.CloseOdevec(ode)
