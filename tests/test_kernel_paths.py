@@ -33,7 +33,7 @@ def _oracle(O, wl, group=None, **kw):
 
 def _same(g, o):
     for name, a, b in zip(("y", "t", "dt", "status", "stats"), g, o):
-        assert np.array_equal(a, b), "%s differs in %d places" % (name, int(np.sum(np.asarray(a) != np.asarray(b))))
+        assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f"), "%s differs in %d places" % (name, int(np.sum(np.asarray(a) != np.asarray(b))))
 
 
 def test_rate_table_sizes(gpu_lib, oracle):
