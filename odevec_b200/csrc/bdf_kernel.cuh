@@ -1871,19 +1871,36 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
         cached_grid = sms * (per_sm > 0 ? per_sm : 1);
     }
     const int nnz[] = {Nets::NNZ...};
+    const bool block[] = {MultiJob<Nets, LUT>::BLOCK...};
+    /* Blocks of each job: first a block per 32 cells for the large networks
+       (all but one per other job at most), whose cells take longest from
+       start to end; the rest in proportion to cells times LU entries, an
+       estimate of the work.  At least one per job. */
+    int nb[MULTI_MAX_JOBS];
+    int left = cached_grid;
     double total = 0.0;
-    for (int j = 0; j < P.njobs; ++j)
-        total += (double)P.job[j].ncells * nnz[P.net[j]];
-    int grid = cached_grid;
-    if (grid < P.njobs)
-        grid = P.njobs;
+    for (int j = 0; j < P.njobs; ++j) {
+        nb[j] = 1;
+        --left;
+        if (!block[P.net[j]])
+            total += (double)P.job[j].ncells * nnz[P.net[j]];
+    }
+    for (int j = 0; j < P.njobs && left > 0; ++j)
+        if (block[P.net[j]]) {
+            const int64_t want = (P.job[j].ncells + 31) / 32 - 1;
+            const int more = (int)(want < left ? want : left);
+            if (more > 0) {
+                nb[j] += more;
+                left -= more;
+            }
+        }
+    for (int j = 0; j < P.njobs && left > 0; ++j)
+        if (!block[P.net[j]] && total > 0.0)
+            nb[j] += (int)(left * ((double)P.job[j].ncells * nnz[P.net[j]]) / total);
     int start = 0;
     for (int j = 0; j < P.njobs; ++j) {
         P.block_start[j] = start;
-        int nb = total > 0.0 ? (int)(grid * ((double)P.job[j].ncells * nnz[P.net[j]]) / total) : 0;
-        if (nb < 1)
-            nb = 1;
-        start += nb;
+        start += nb[j];
     }
     P.block_start[P.njobs] = start;
     kern<<<start, MULTI_BS, smem, stream>>>(P);
