@@ -48,6 +48,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <type_traits>
 
 #include "../../include/odevec_b200.h"
@@ -319,6 +320,11 @@ template <> struct StageCfg<20> { static constexpr int SHM = 4; static constexpr
    warps in soft lockstep (where three blocks' histories fit an SM: up to 12
    solver species) */
 template <> struct StageCfg<21> { static constexpr int SHM = 2; static constexpr bool SOFT = true;  static constexpr int BS = 128, MINB = 3, REFILL = 16, PERIOD = 4; };
+
+/* not a caller's choice: the shape of stagings 3 and 9 for few cells (see
+   launch) -- as 2 with the block's four warps in soft lockstep */
+constexpr int SPREAD_STAGE = 22;
+template <> struct StageCfg<22> { static constexpr int SHM = 1; static constexpr bool SOFT = true;  static constexpr int BS = 128, MINB = 1, REFILL = 16, PERIOD = 4; };
 
 /* Soft lockstep.  The warps of a block wait for each other at the top of
    every trip of the cell loop, so they run the same phase code at the same
@@ -1676,24 +1682,51 @@ cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream
     const bool chosen = block > 0 || grid > 0; /* the caller fixes the shape */
     if (Cfg::SHM || block <= 0 || block > Cfg::BS)
         block = Cfg::BS;
-    static int cached_grid[2] = {0, 0};
-    static int cached_sms = 0;
-    if (cached_grid[0] == 0 || cached_grid[1] != block) {
+    /* the device's SMs and the resident blocks of this block size, packed into
+       one word so that threads that launch for the first time together read
+       all of it or nothing */
+    static std::atomic<unsigned long long> cached{0ull};
+    unsigned long long word = cached.load();
+    if (word >> 48 != (unsigned long long)block) {
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
-        if (smem > 48 * 1024) {
+        if (smem > 40 * 1024) { /* the default 48 KB hold the lockstep words too */
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess)
                 return e;
         }
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem);
-        cached_grid[0] = sms * (per_sm > 0 ? per_sm : 1);
-        cached_grid[1] = block;
-        cached_sms = sms;
+        if (sms <= 0)
+            return cudaErrorInvalidDevice;
+        word = (unsigned long long)block << 48 | (unsigned long long)sms << 24 |
+               (unsigned long long)(sms * (per_sm > 0 ? per_sm : 1));
+        cached.store(word);
     }
+    const int sms = (int)(word >> 24 & 0xffffffu), resident = (int)(word & 0xffffffu);
     LaunchArgs b = a;
-    if (Net::ND <= 32 && !chosen && a.ncells <= (int64_t)cached_sms * SPREAD_WARPS * 32) {
+    if constexpr (G == 1 && (STAGE == 3 || STAGE == 9) && Net::ND > 4 && Net::ND <= 32 &&
+                  Staging<Net, LUT, 1, StageCfg<SPREAD_STAGE>::BS>::smem_bytes <= 226 * 1024) {
+        /* Up to a few cells per lane of four warps per SM, the factors go into
+           shared memory beside the history: with four warps they fit, and a
+           trip then reads nothing but on-chip memory.  PRIMORDIAL, against
+           staging 9: FP64 1,000 cells 7.0 -> 5.6 ms, 8,192 cells 10.3 -> 8.0,
+           18,944 cells 11.2 -> 8.7, 32,000 cells 13.7 -> 10.6, 75,776 cells
+           16.0 -> 15.6, 100,003 cells 18.9 -> 19.6; FP32-LU 1,000 cells 4.9 ->
+           4.4 ms, 18,944 cells 7.1 -> 6.8, 56,832 cells 10.3 -> 9.9, 75,776
+           cells 11.1 -> 12.2.  So the line lies at 4 cells per lane in FP64
+           and 3 with FP32 factors.  Continued solves are short and gain more
+           from a lane's shorter trip: 8 in FP64 (one step with contraction,
+           100,003 cells 2.23 -> 1.99 ms, 150,001 cells 2.67 -> 2.46, 1,000,000
+           cells equal).  Without the lockstep 8,192 cells take 8.5 instead of
+           8.0 ms, 18,000 cells 9.8 instead of 8.4.  Up to four species the
+           history is in registers instead. */
+        const int64_t lanes = (int64_t)sms * SPREAD_WARPS * 32;
+        const int per_lane = sizeof(LUT) == 8 ? (a.resume == 1 ? 8 : 4) : 3;
+        if (!chosen && a.ncells <= lanes * per_lane)
+            return launch<Net, G, LUT, SPREAD_STAGE>(a, 0, 0, stream);
+    }
+    if (Net::ND <= 32 && !chosen && a.ncells <= (int64_t)sms * SPREAD_WARPS * 32) {
         /* Few cells: over all SMs, at most one warp per scheduler and only as
            many lanes per warp as that takes.  The time is that of the longest
            cells' chain of steps then, and a warp's trip is the shorter the
@@ -1707,12 +1740,12 @@ cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream
            cells: 186 ms spread, 168 ms in 256-cell blocks). */
         int64_t groups, lanes = 1; /* work items: cells, or lockstep groups (a warp each) */
         groups = G == 1 ? a.ncells : (a.ncells + 31) / 32;
-        int64_t warps = (groups + cached_sms - 1) / cached_sms; /* per SM */
+        int64_t warps = (groups + sms - 1) / sms; /* per SM */
         const int64_t most = Cfg::BS / 32 < SPREAD_WARPS ? Cfg::BS / 32 : SPREAD_WARPS;
         if (warps > most)
             warps = most;
         if (G == 1)
-            lanes = (groups + cached_sms * warps - 1) / (cached_sms * warps);
+            lanes = (groups + sms * warps - 1) / (sms * warps);
         b.lanes = (int32_t)(lanes < 32 ? lanes : 32);
         block = (int)(32 * warps);
         const int64_t per_block = warps * (G == 1 ? (int64_t)b.lanes : 1);
@@ -1720,7 +1753,7 @@ cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream
         if (grid < 1)
             grid = 1;
     } else if (grid <= 0) {
-        grid = cached_grid[0];
+        grid = resident;
         const int64_t warps_needed = (a.ncells + 31) / 32;
         const int64_t blocks_needed = (warps_needed * 32 + block - 1) / block;
         if (blocks_needed < grid)
@@ -1857,8 +1890,9 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
     auto kern = bdf_multi_kernel<LUT, Nets...>;
     constexpr size_t smem = multi_smem_bytes<LUT, Nets...>();
     static_assert(smem <= 226 * 1024, "the set's largest state vectors exceed a block's shared memory");
-    static int cached_grid = 0;
-    if (cached_grid == 0) {
+    static std::atomic<int> cached{0};
+    int resident = cached.load();
+    if (resident == 0) {
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
         if (smem > 48 * 1024) {
@@ -1868,7 +1902,8 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
         }
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MULTI_BS, smem);
-        cached_grid = sms * (per_sm > 0 ? per_sm : 1);
+        resident = sms * (per_sm > 0 ? per_sm : 1);
+        cached.store(resident);
     }
     const int nnz[] = {Nets::NNZ...};
     const bool block[] = {MultiJob<Nets, LUT>::BLOCK...};
@@ -1877,7 +1912,7 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
        start to end; the rest in proportion to cells times LU entries, an
        estimate of the work.  At least one per job. */
     int nb[MULTI_MAX_JOBS];
-    int left = cached_grid;
+    int left = resident;
     double total = 0.0;
     for (int j = 0; j < P.njobs; ++j) {
         nb[j] = 1;

@@ -895,22 +895,25 @@ cudaError_t launch_blk(const LaunchArgs& a, int grid, cudaStream_t stream)
 {
     auto kern = blk_kernel<Net, LUT>;
     constexpr size_t smem = BlkLayout<Net, LUT>::smem_bytes;
-    static int cached_sms = 0;
-    if (cached_sms == 0) {
-        int dev = 0, sms = 0;
+    static std::atomic<int> cached{0};
+    int sms = cached.load();
+    if (sms == 0) {
+        int dev = 0;
         cudaGetDevice(&dev);
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess)
             return e;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cached_sms = sms;
+        if (sms <= 0)
+            return cudaErrorInvalidDevice;
+        cached.store(sms);
     }
     LaunchArgs b = a;
     if (grid <= 0) {
-        int64_t lanes = (a.ncells + cached_sms - 1) / cached_sms;
+        int64_t lanes = (a.ncells + sms - 1) / sms;
         b.lanes = (int32_t)(lanes < 32 ? lanes : 32);
         const int64_t want = (a.ncells + b.lanes - 1) / b.lanes;
-        grid = (int)(want < cached_sms ? want : cached_sms);
+        grid = (int)(want < sms ? want : sms);
     }
     kern<<<grid, 32 * BLK_WARPS, smem, stream>>>(b);
     return cudaGetLastError();

@@ -130,16 +130,21 @@ int32_t fail(int32_t code, const char* fmt, ...)
     return code;
 }
 
-/* automatic staging (the measured best on B200 without a tuning table):
-   thread-local arrays, 3 blocks of 128 threads per SM for per-cell control
-   up to 32 solver-state species, 2 blocks above (more registers per cell),
-   2 blocks for lockstep groups.  The warp-per-cell staging (7) is slower on
-   the shipped networks and is only used when asked for. */
+/* automatic staging (the measured best on B200 without a tuning table): for
+   per-cell control soft lockstep with the history in shared memory (9) from 5
+   to 16 solver-state species, whose history fits a block (131,072 cells, FP64,
+   against staging 3: PRIMORDIAL dense 66 -> 28 ms, CMK-ordered 51 -> 22 ms,
+   difference quotients 107 -> 44 ms, the heating/cooling network 109 -> 67
+   ms); thread-local arrays in 3 blocks of 128 threads per SM otherwise up to
+   32 species, 2 blocks above (more registers per cell); 2 blocks for lockstep
+   groups.  The warp-per-cell staging (7) is slower on the shipped networks and
+   is only used when asked for. */
 int auto_staging(const NetEntry& e, int group_size)
 {
     if (group_size != 1)
         return 1;
-    return e.sizes[5] > 32 ? 1 : 3;
+    const int nd = e.sizes[5];
+    return nd > 32 ? 1 : (nd > 4 && nd <= 16 ? 9 : 3);
 }
 
 int find_net(const char* tag)

@@ -139,7 +139,8 @@ def network_info(tag):
 
 
 # resident blocks per SM of each staging (block size x blocks: the launch
-# shape the kernel is compiled for; 0 = the library's automatic choice, 3)
+# shape the kernel is compiled for; 0 = the library's automatic choice, 3 where
+# the largest of its choices is meant)
 BLOCKS_PER_SM = {0: 3, 1: 2, 2: 1, 3: 3, 4: 4, 5: 1, 6: 1, 7: 3, 8: 1, 9: 1, 10: 1, 11: 1, 12: 1, 13: 2, 14: 1, 15: 1, 16: 1, 17: 1, 18: 1, 19: 1, 20: 3, 21: 3}
 # cells one block of each staging holds at a time (thread per cell: the block
 # size; 32, 16 or 8 lanes per cell: 8, 16 or 32 cells in 8 warps; staging 18

@@ -177,3 +177,33 @@ def test_small_network_far_operands(gpu_lib, oracle, group, scale):
         _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl, group=group, max_attempts=3000))
     finally:
         gpu_lib.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("network", ["PRIMORDIAL_CSC_FF", "PRIMORDIAL_DENSE_NONE"])
+@pytest.mark.parametrize("n", [1, 593, 18944, 18945])
+def test_few_cells_on_chip(gpu_lib, oracle, network, n):
+    """The shape of solves of few cells with the factors in shared memory: one
+    lane, several lanes per warp, every lane once, and lanes that take a second
+    cell."""
+    wl = W.primordial(ncells=n, seed=6, network=network)
+    wl.t_stop[:] = 1e8
+    ode = _solver(gpu_lib, wl)
+    try:
+        _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl))
+    finally:
+        gpu_lib.CloseOdevec(ode)
+
+
+def test_few_cells_fp32_factors(gpu_lib):
+    """FP32 factors of every network above four species: the same bits as in a
+    shape that the caller fixes."""
+    for wl in (W.hctoy(ncells=700, seed=3), W.primordial(ncells=700, seed=3)):
+        wl.t_stop[:] = 1e8
+        got = []
+        for kw in ({}, {"staging": 3, "grid_blocks": 40}):
+            ode = _solver(gpu_lib, wl, precision="fp32_lu", escalation=False, **kw)
+            try:
+                got.append(_gpu(gpu_lib, ode, wl))
+            finally:
+                gpu_lib.CloseOdevec(ode)
+        _same(got[0], got[1])
