@@ -2005,6 +2005,11 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
                 OV_STAGE_CASE(NET, double, 15)                                               \
                 OV_STAGE_CASE(NET, double, 16)                                               \
                 if constexpr (blk_ok<NET, double>()) {                                       \
+                    if constexpr (BLK_SPLIT && y_fits<NET, 256>()) {                         \
+                        if (a.ncells >= BLK_SPLIT_CELLS) {                                   \
+                            OV_STAGE_CASE(NET, double, 18)                                   \
+                        }                                                                    \
+                    }                                                                        \
                     if (stage == 18)                                                         \
                         return launch_blk<NET, double>(a, grid, s);                          \
                 } else if constexpr (y_fits<NET, 256>()) {                                   \

@@ -54,6 +54,15 @@ constexpr bool BLK_SPLIT = false;
 constexpr bool BLK_SPLIT = true;
 #endif
 
+/* Without contraction a thread per cell (staging 18's other form) is the faster
+   one from two cells per lane on, 256 lanes on each of 148 SMs: its divisions
+   run for 32 cells beside seven other warps' work, here in one warp while the
+   others wait.  SYN64 FP64, thread per cell / block per 32 cells: 37,888
+   cells 290 / 302 ms, 65,536 cells 526 / 521, 75,776 cells 560 / 599,
+   262,144 cells 1,810 / 2,060; 3,001 cells 157 / 38.  (With contraction
+   262,144 cells take 1,624 ms here against 1,910, FP32-LU 944 against 1,530.) */
+constexpr int64_t BLK_SPLIT_CELLS = 2 * 148 * 256;
+
 template <class Net, class LUT>
 struct BlkLayout {
     static constexpr int ND = Net::ND;

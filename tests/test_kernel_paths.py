@@ -207,3 +207,16 @@ def test_few_cells_fp32_factors(gpu_lib):
             finally:
                 gpu_lib.CloseOdevec(ode)
         _same(got[0], got[1])
+
+
+@pytest.mark.parametrize("n", [75775, 75776])
+def test_block_kernel_limit(gpu_lib, oracle, n):
+    """The last cell count of the block kernel in FP64 and the first of a thread
+    per cell."""
+    wl = W.syn64(ncells=n, seed=12)
+    wl.t_stop[:] = 1e-6
+    ode = _solver(gpu_lib, wl)
+    try:
+        _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl))
+    finally:
+        gpu_lib.CloseOdevec(ode)
