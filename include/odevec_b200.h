@@ -110,8 +110,8 @@ typedef struct odevec_opts {
        memory, 20 = as 3 with the state vector in shared memory (18-20:
        networks above 32 solver species; 18 is one block of eight warps per
        32 cells, which share a cell's species, for constant-coefficient
-       networks of up to 64 species in CSC or DENSE packaging with the
-       symbolic Jacobian); 21 = as 3 with the history in
+       networks of up to 64 species with the symbolic Jacobian, and for solves
+       in FP64 without contraction below 75,776 cells); 21 = as 3 with the history in
        shared memory and each block in soft lockstep (up to 12 solver
        species) (2-21: per-cell control only).  In 2-6 and 8-16 idle lanes take new cells on every
        16th trip of the cell loop (17: every 32nd), so cells are set up

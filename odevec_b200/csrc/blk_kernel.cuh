@@ -25,7 +25,7 @@
  * line network code, most of it in one warp at a time (about 16 cycles per
  * instruction in the solve, the right-hand side and the factorisation); no
  * memory traffic to speak of.  SYN64 against a thread per cell in
- * 256-thread blocks with the state in shared memory, B200: 65,536 cells FP32-LU 451 -> 245 ms, FP64 575 -> 497 ms, FP64 with
+ * 256-thread blocks with the state in shared memory, B200: 65,536 cells FP32-LU 451 -> 245 ms, FP64 575 -> 515 ms, FP64 with
  * contraction 511 -> 428 ms; 3,001 cells FP32-LU 130 -> 25 ms, FP64 157 -> 38
  * ms; 64 cells FP64 121 -> 18 ms.
  *
