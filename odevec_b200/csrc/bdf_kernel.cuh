@@ -888,8 +888,11 @@ struct Cell {
                 if (!ieee) {
                     unsigned bad = 0u;
                     Net::template lu_factor<LUT>(PivotLU<Net, decltype(a)>{a, rp, &bad});
-                    if (bad) {
-                        ieee = true; /* once more from the matrix */
+                    /* once more from the matrix: the whole lockstep group,
+                       whose difference quotients take a norm over the group
+                       (the same values either way) */
+                    if (group_any<G>(bad != 0u)) {
+                        ieee = true;
                         continue;
                     }
                     break;

@@ -220,3 +220,21 @@ def test_block_kernel_limit(gpu_lib, oracle, n):
         _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl))
     finally:
         gpu_lib.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("far", ["tiny", "nan", "masked"])
+def test_lockstep_difference_quotients_far_operands(gpu_lib, oracle, far):
+    """A lockstep group of a small network with difference quotients, one cell
+    of which needs IEEE divisions: the whole group forms its matrix again (the
+    quotients take a norm over the group), an ordinary group beside it does
+    not."""
+    wl = W.rober(ncells=64, seed=8, network="ROBER_DENSE_NONE_LU3")
+    wl.y[:, 5] = (1e-290, 1e-295, 0.0) if far == "tiny" else np.nan
+    wl.t_stop[:] = 1e2
+    mask = np.ones(64, dtype=bool)
+    mask[5] = far != "masked"
+    ode = _solver(gpu_lib, wl, max_attempts=3000)
+    try:
+        _same(_gpu(gpu_lib, ode, wl, mask), _oracle(oracle, wl, max_attempts=3000, mask=mask))
+    finally:
+        gpu_lib.CloseOdevec(ode)
