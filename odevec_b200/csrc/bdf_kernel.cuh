@@ -48,11 +48,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <atomic>
 #include <type_traits>
 
 #include "../../include/odevec_b200.h"
 #include "ov_common.h"
+#include "ov_host.h"
 #include "ov_launch.h"
 #include "rates_primordial.h"
 
@@ -1685,28 +1685,15 @@ cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream
     const bool chosen = block > 0 || grid > 0; /* the caller fixes the shape */
     if (Cfg::SHM || block <= 0 || block > Cfg::BS)
         block = Cfg::BS;
-    /* the device's SMs and the resident blocks of this block size, packed into
-       one word so that threads that launch for the first time together read
-       all of it or nothing */
-    static std::atomic<unsigned long long> cached{0ull};
-    unsigned long long word = cached.load();
-    if (word >> 48 != (unsigned long long)block) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        if (smem > 40 * 1024) { /* the default 48 KB hold the lockstep words too */
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess)
-                return e;
-        }
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem);
-        if (sms <= 0)
-            return cudaErrorInvalidDevice;
-        word = (unsigned long long)block << 48 | (unsigned long long)sms << 24 |
-               (unsigned long long)(sms * (per_sm > 0 ? per_sm : 1));
-        cached.store(word);
-    }
-    const int sms = (int)(word >> 24 & 0xffffffu), resident = (int)(word & 0xffffffu);
+    static Residency residency;
+    int sms = 0, resident = 0;
+    cudaError_t err = device_sms(&sms);
+    if (err == cudaSuccess)
+        err = allow_smem((const void*)kern, smem);
+    if (err == cudaSuccess)
+        err = resident_blocks(residency, (const void*)kern, block, smem, &resident);
+    if (err != cudaSuccess)
+        return err;
     LaunchArgs b = a;
     if constexpr (G == 1 && (STAGE == 3 || STAGE == 9) && Net::ND > 4 && Net::ND <= 32 &&
                   Staging<Net, LUT, 1, StageCfg<SPREAD_STAGE>::BS>::smem_bytes <= 226 * 1024) {
@@ -1893,21 +1880,13 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
     auto kern = bdf_multi_kernel<LUT, Nets...>;
     constexpr size_t smem = multi_smem_bytes<LUT, Nets...>();
     static_assert(smem <= 226 * 1024, "the set's largest state vectors exceed a block's shared memory");
-    static std::atomic<int> cached{0};
-    int resident = cached.load();
-    if (resident == 0) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess)
-                return e;
-        }
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MULTI_BS, smem);
-        resident = sms * (per_sm > 0 ? per_sm : 1);
-        cached.store(resident);
-    }
+    static Residency residency;
+    int resident = 0;
+    cudaError_t err = allow_smem((const void*)kern, smem);
+    if (err == cudaSuccess)
+        err = resident_blocks(residency, (const void*)kern, MULTI_BS, smem, &resident);
+    if (err != cudaSuccess)
+        return err;
     const int nnz[] = {Nets::NNZ...};
     const bool block[] = {MultiJob<Nets, LUT>::BLOCK...};
     /* Blocks of each job: first a block per 32 cells for the large networks

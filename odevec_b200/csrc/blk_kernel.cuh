@@ -904,19 +904,12 @@ cudaError_t launch_blk(const LaunchArgs& a, int grid, cudaStream_t stream)
 {
     auto kern = blk_kernel<Net, LUT>;
     constexpr size_t smem = BlkLayout<Net, LUT>::smem_bytes;
-    static std::atomic<int> cached{0};
-    int sms = cached.load();
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess)
-            return e;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0)
-            return cudaErrorInvalidDevice;
-        cached.store(sms);
-    }
+    int sms = 0;
+    cudaError_t err = device_sms(&sms);
+    if (err == cudaSuccess)
+        err = allow_smem((const void*)kern, smem);
+    if (err != cudaSuccess)
+        return err;
     LaunchArgs b = a;
     if (grid <= 0) {
         int64_t lanes = (a.ncells + sms - 1) / sms;

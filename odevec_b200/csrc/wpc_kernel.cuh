@@ -897,22 +897,15 @@ cudaError_t launch_wpc(const LaunchArgs& a, int grid, cudaStream_t stream)
     using L = WpcLayout<Net, LUT, K>;
     auto kern = wpc_kernel<Net, LUT, K>;
     constexpr int block = 32 * L::WARPS;
-    static int cached = 0;
-    if (cached == 0) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        if (L::block_bytes > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)L::block_bytes);
-            if (e != cudaSuccess)
-                return e;
-        }
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, L::block_bytes);
-        cached = sms * (per_sm > 0 ? per_sm : 1);
-    }
+    static Residency residency;
+    int resident = 0;
+    cudaError_t err = allow_smem((const void*)kern, L::block_bytes);
+    if (err == cudaSuccess)
+        err = resident_blocks(residency, (const void*)kern, block, L::block_bytes, &resident);
+    if (err != cudaSuccess)
+        return err;
     if (grid <= 0) {
-        grid = cached;
+        grid = resident;
         const int64_t blocks_needed = (a.ncells + L::GROUPS - 1) / L::GROUPS;
         if (blocks_needed < grid)
             grid = (int)blocks_needed;
