@@ -238,3 +238,108 @@ def test_lockstep_difference_quotients_far_operands(gpu_lib, oracle, far):
         _same(_gpu(gpu_lib, ode, wl, mask), _oracle(oracle, wl, max_attempts=3000, mask=mask))
     finally:
         gpu_lib.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("options", [dict(max_attempts=40), dict(CheckNegatives=True), dict(fix_restart=True)])
+def test_block_kernel_exits(gpu_lib, oracle, options):
+    """The block kernel's ways out of a cell, and its restarts at order 1: cells
+    out of attempts, steps below dt_min after a negative prediction and after a
+    Newton failure (a NaN and an infinite state), beside ordinary cells."""
+    wl = W.syn64(ncells=70, seed=4)
+    wl.t_stop[:] = 10.0 ** np.random.default_rng(2).uniform(-3.0, 3.0, 70)
+    wl.y[7, 3], wl.y[5, 40], wl.y[9, 66] = np.nan, -1e-3, np.inf
+    ode = _solver(gpu_lib, wl, staging=18, **options)
+    try:
+        kw = {"check_negatives" if k == "CheckNegatives" else k: v for k, v in options.items()}
+        _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl, **kw))
+    finally:
+        gpu_lib.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("precision,max_attempts", [("fp64", 0), ("fp32_lu", 0), ("fp32_lu", 5)])
+def test_block_kernel_yields(gpu_lib, precision, max_attempts):
+    """The block kernel stops starting cells, and continuations start the rest,
+    the escalation of failed cells (with five attempts: all of them) included:
+    the bits of one uninterrupted solve.  More cells than all blocks hold."""
+    import torch
+    S = gpu_lib
+    n = 6000
+    wl = W.syn64(ncells=n, seed=5)
+    wl.t_stop[:] = 1e2
+    got = []
+    for yielding in (False, True):
+        ode = _solver(S, wl, precision=precision, max_attempts=max_attempts)
+        try:
+            y, t, d, ts = (torch.tensor(a, device="cuda") for a in (wl.y, wl.t0, wl.dt0, wl.t_stop))
+            st = torch.zeros(n, dtype=torch.int32, device="cuda")
+            flag = torch.ones(1, dtype=torch.int32, device="cuda")
+            S.set_yield(ode, flag if yielding else None)
+            S.SolveODERange(ode, 0, n, t, d, ts, y, st)
+            if yielding:
+                assert S.cells_started(ode) < n
+                for _ in range(20):
+                    S.SolveODERange(ode, 0, n, t, d, ts, y, st, cont=True)
+                    if S.cells_started(ode) >= n:
+                        break
+                S.set_yield(ode, None)
+            torch.cuda.synchronize()
+            got.append([a.cpu().numpy() for a in (y, t, d, st)])
+        finally:
+            S.CloseOdevec(ode)
+    _same(got[1], got[0])
+    assert np.all(got[0][3] == (4 if max_attempts else 0))
+
+
+@pytest.mark.parametrize("cells", [(4096, 5000, 40), (33, 70, 700)])
+def test_multi_block_jobs_fp32_factors(gpu_lib, cells):
+    """FP32 factors in one launch whose blocks go from one job's kernel to
+    another's: the bits of separate solves."""
+    import torch
+    from odevec_b200.multi import SolveMany
+    S = gpu_lib
+    got = []
+    for fused in (True, False):
+        wls = [W.rober(cells[0], seed=2), W.primordial(cells[1], seed=2), W.syn64(cells[2], seed=2)]
+        wls[2].t_stop[:] = 1e2
+        odes, jobs = [], []
+        for wl in wls:
+            odes.append(_solver(S, wl, nvector=1, precision="fp32_lu", escalation=False))
+            jobs.append((odes[-1], *[torch.tensor(a, device="cuda") for a in (wl.t0, wl.dt0, wl.t_stop, wl.y)]))
+        try:
+            if fused:
+                SolveMany(jobs, fused=True).run()
+            else:
+                for ode, t, d, ts, y in jobs:
+                    S.SolveODE(ode, t, d, ts, y)
+            torch.cuda.synchronize()
+            got.append([a.cpu().numpy() for ode, t, d, ts, y in jobs for a in (y, t, d, ode.status)])
+        finally:
+            for ode in odes:
+                S.CloseOdevec(ode)
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision,cells", [("fp64", 700), ("fp64", 151552), ("fp64", 151553), ("fp32_lu", 56833)])
+def test_resumed_on_chip(gpu_lib, precision, cells):
+    """A solve and its continuation at the sizes where either leaves the shape
+    with the factors on chip: state and statistics as in a shape
+    that the caller fixes."""
+    import torch
+    S = gpu_lib
+    wl = W.primordial(ncells=cells, seed=6)
+    wl.t_stop[:] = 1e6
+    got = []
+    for kw in ({}, {"staging": 9, "grid_blocks": 148}):
+        ode = _solver(S, wl, precision=precision, escalation=False, **kw)
+        try:
+            y, t, d = (torch.tensor(a, device="cuda") for a in (wl.y, wl.t0, wl.dt0))
+            ws = S.Workspace(ode, cells)
+            for k in (1, 2):
+                t, d = S.SolveODE(ode, t, d, torch.tensor(wl.t_stop * k, device="cuda"), y, workspace=ws,
+                                  resume=k > 1)
+            torch.cuda.synchronize()
+            got.append([a.cpu().numpy() for a in (y, t, d, ode.status, ode.stats)])
+        finally:
+            S.CloseOdevec(ode)
+    _same(got[0], got[1])
