@@ -191,12 +191,10 @@ struct odevec_solver {
     /* rate tables ([cells][reactions], networks with rate coefficients): the
        last one is in use, of rate_cells cells; smaller ones before it stay
        until odevec_close, since a captured graph may hold their address.
-       Each is at least twice the one before it.  rate_cur: that of the last
-       solve, or null (a continuation reuses it) */
+       Each is at least twice the one before it */
     int64_t rate_cells;
     int rate_ntabs;
     double* rate_tabs[OV_RATE_TABS];
-    double* rate_cur;
 };
 /* d_queue words: [0] the solve's work counter, [1] cells that failed with
    FP32 factors, [2] the FP64 re-solve's work counter */
@@ -568,10 +566,13 @@ static int32_t visit_order(odevec_solver* s, int64_t ncells, const double* t, co
    Evaluated in the solve kernel as each cell is set up, the same laws run
    for the two or three lanes of a warp that take a cell at the same time.
    Without a table (no room for it, a capture that would have to allocate it,
-   or few cells) the solve kernel evaluates them, with the same results. */
+   or few cells) the solve kernel evaluates them, with the same results.  A
+   continuation fills it again (no solve changes the temperature): the solve it
+   continues may be a replayed graph with another table, or other cells may
+   have been solved since. */
 static cudaError_t rate_table(odevec_solver* s, ov::LaunchArgs& a, ov::launch_fn fn, cudaStream_t st)
 {
-    a.rates = s->rate_cur = nullptr;
+    a.rates = nullptr;
     const int64_t nrea = g_nets[s->net].sizes[2];
     if (nrea <= 0 || a.ncells < OV_RATES_MIN_CELLS)
         return cudaSuccess;
@@ -592,10 +593,7 @@ static cudaError_t rate_table(odevec_solver* s, ov::LaunchArgs& a, ov::launch_fn
         s->rate_cells = cells;
     }
     a.rates = s->rate_tabs[s->rate_ntabs - 1];
-    const cudaError_t e = fn(a, 1, 0, ov::STAGE_RATES, 0, 0, st);
-    if (e == cudaSuccess)
-        s->rate_cur = a.rates;
-    return e;
+    return fn(a, 1, 0, ov::STAGE_RATES, 0, 0, st);
 }
 
 static int32_t solve_impl(odevec_solver* s, int64_t ncells, int64_t stride, double* y, double* t,
@@ -643,7 +641,7 @@ static int32_t solve_impl(odevec_solver* s, int64_t ncells, int64_t stride, doub
     a.save_y = a.save_t = a.save_dt = nullptr;
     a.yield = s->yield;
     a.order = nullptr;
-    a.rates = cont ? s->rate_cur : nullptr;
+    a.rates = nullptr;
     a.lanes = 0;
     cudaStream_t st = (cudaStream_t)stream;
     /* a continuation keeps the work counter (and the failure count) of the
@@ -706,8 +704,7 @@ static int32_t solve_impl(odevec_solver* s, int64_t ncells, int64_t stride, doub
         if (!a.status)
             a.status = s->fb_status;
     }
-    if (!cont)
-        err = rate_table(s, a, fn, st);
+    err = rate_table(s, a, fn, st);
     if (err == cudaSuccess)
         err = fn(a, o.group_size, lu, stage, o.block_threads, o.grid_blocks, st);
     if (escalate && err == cudaSuccess) {

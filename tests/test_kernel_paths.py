@@ -343,3 +343,39 @@ def test_resumed_on_chip(gpu_lib, precision, cells):
         finally:
             S.CloseOdevec(ode)
     _same(got[0], got[1])
+
+
+def test_continuation_of_a_replayed_solve(gpu_lib, oracle):
+    """A captured solve yields and is continued after another solve on the same
+    solver, whose rate table is a larger one: the continuation takes the rates
+    of its own cells."""
+    import torch
+    S = gpu_lib
+    a, b = W.primordial(ncells=20000, seed=31), W.primordial(ncells=30000, seed=32)
+    for wl in (a, b):
+        wl.t_stop[:] = 1e6
+    ode = _solver(S, a)
+    try:
+        flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+        S.set_yield(ode, flag)
+        y, t, d, ts = (torch.tensor(v, device="cuda") for v in (a.y, a.t0, a.dt0, a.t_stop))
+        init = [v.clone() for v in (y, t, d)]
+        st = torch.zeros(a.ncells, dtype=torch.int32, device="cuda")
+        S.SolveODERange(ode, 0, a.ncells, t, d, ts, y, st) # sizes the table
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            S.SolveODERange(ode, 0, a.ncells, t, d, ts, y, st)
+        _same(_gpu(S, ode, b), _oracle(oracle, b))
+        for v, v0 in zip((y, t, d), init):
+            v.copy_(v0)
+        flag.fill_(1)
+        g.replay()
+        assert S.cells_started(ode) < a.ncells
+        flag.zero_()
+        S.SolveODERange(ode, 0, a.ncells, t, d, ts, y, st, cont=True)
+        torch.cuda.synchronize()
+        _same([v.cpu().numpy() for v in (y, t, d, st)], _oracle(oracle, a)[:4])
+        S.set_yield(ode, None)
+    finally:
+        S.CloseOdevec(ode)
