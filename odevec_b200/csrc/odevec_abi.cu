@@ -187,7 +187,8 @@ struct odevec_solver {
     int32_t* ord_vals;
     void* ord_temp;
     size_t ord_temp_bytes;
-    const int32_t* ord_cur;
+    const int32_t* ord_cur; /* the last order computed, of ord_n cells */
+    int64_t ord_n;
     /* rate tables ([cells][reactions], networks with rate coefficients): the
        last one is in use, of rate_cells cells; smaller ones before it stay
        until odevec_close, since a captured graph may hold their address.
@@ -517,12 +518,11 @@ int32_t odevec_cells_started(odevec_solver* s, void* stream, int64_t* started)
 /* The visit order of a per-cell solve of ncells cells (device arrays t,
    t_stop): cells with the longest integration span first, computed on
    `st` into s's buffers (*order = null below OV_ORDER_MIN_CELLS cells);
-   remembered as s->ord_cur for a continuation. */
+   remembered for a continuation. */
 static int32_t visit_order(odevec_solver* s, int64_t ncells, const double* t, const double* t_stop,
                            cudaStream_t st, const int32_t** order)
 {
     *order = nullptr;
-    s->ord_cur = nullptr;
     if (ncells < OV_ORDER_MIN_CELLS || ncells > (int64_t)INT32_MAX)
         return OV_API_OK;
     cudaError_t err = cudaSuccess;
@@ -531,6 +531,8 @@ static int32_t visit_order(odevec_solver* s, int64_t ncells, const double* t, co
         s->ord_keys = nullptr; s->ord_vals = nullptr; s->ord_temp = nullptr;
         s->ord_cells = 0;
         s->ord_temp_bytes = 0;
+        s->ord_cur = nullptr;
+        s->ord_n = 0;
         const size_t n = (size_t)ncells;
         err = cudaMalloc(&s->ord_keys, 2 * n * sizeof(uint16_t));
         if (err == cudaSuccess) err = cudaMalloc(&s->ord_vals, 2 * n * sizeof(int32_t));
@@ -557,6 +559,7 @@ static int32_t visit_order(odevec_solver* s, int64_t ncells, const double* t, co
     if (err != cudaSuccess)
         return fail(OV_API_ECUDA, "odevec_solve: visit order: %s", cudaGetErrorString(err));
     s->ord_cur = vb.Current();
+    s->ord_n = ncells;
     *order = s->ord_cur;
     return OV_API_OK;
 }
@@ -657,13 +660,14 @@ static int32_t solve_impl(odevec_solver* s, int64_t ncells, int64_t stride, doub
        on PRIMORDIAL that costs about what the order gains with FP32
        factors, and gains 3 % in FP64.) */
     if (cont) {
-        a.order = s->ord_cur;
+        /* not the order of another count: the solve continued may be a
+           replayed graph, and other cells may have been solved since */
+        if (o.group_size == 1 && s->ord_n == ncells)
+            a.order = s->ord_cur;
     } else if (o.group_size == 1) {
         const int32_t rc = visit_order(s, ncells, t, t_stop, st, &a.order);
         if (rc)
             return rc;
-    } else {
-        s->ord_cur = nullptr;
     }
     const int lu = o.precision == OV_PREC_FP32_LU ? 1 : 0;
     ov::launch_fn fn = o.precision == OV_PREC_FP64 ? e.exact : e.fma;

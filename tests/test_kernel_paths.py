@@ -345,13 +345,15 @@ def test_resumed_on_chip(gpu_lib, precision, cells):
     _same(got[0], got[1])
 
 
-def test_continuation_of_a_replayed_solve(gpu_lib, oracle):
+@pytest.mark.parametrize("na,nb", [(20000, 30000), (20000, 40000), (80000, 5000)])
+def test_continuation_of_a_replayed_solve(gpu_lib, oracle, na, nb):
     """A captured solve yields and is continued after another solve on the same
-    solver, whose rate table is a larger one: the continuation takes the rates
-    of its own cells."""
+    solver, whose rate table is a larger one, or which has a visit order where
+    the captured one has none, or the other way round: the continuation takes
+    the rates and the order of its own cells."""
     import torch
     S = gpu_lib
-    a, b = W.primordial(ncells=20000, seed=31), W.primordial(ncells=30000, seed=32)
+    a, b = W.primordial(ncells=na, seed=31), W.primordial(ncells=nb, seed=32)
     for wl in (a, b):
         wl.t_stop[:] = 1e6
     ode = _solver(S, a)
