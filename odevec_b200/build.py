@@ -176,7 +176,7 @@ def build(force: bool = False, jobs: int = 0, verbose: bool = False) -> str:
     abi_obj = os.path.join(BUILD, "odevec_abi.o")
     tune_inc = write_tuning_table()
     multi_inc = write_multi_registry()
-    key = _hash_files(hdrs + [abi_src, os.path.join(GEN, "registry.inc"),
+    key = _hash_files(hdrs + [abi_src, os.path.join(CSRC, "rate_tables.hpp"), os.path.join(GEN, "registry.inc"),
                               os.path.join(GEN, "includes_c.inc"), tune_inc, multi_inc] +
                       [os.path.join(GEN, "net_%s.h" % c) for c, _ in variants()], " ".join(COMMON))
     if force or not os.path.exists(abi_obj) or not os.path.exists(abi_obj + ".key") or \

@@ -20,6 +20,7 @@
 
 #include "../../include/odevec_b200.h"
 #include "ov_launch.h"
+#include "rate_tables.hpp"
 #include "gen/includes_c.inc"
 
 /* launchers, one per variant and arithmetic mode (kernels_<cid>_<mode>.cu) */
@@ -159,8 +160,6 @@ int find_net(const char* tag)
 
 }  // namespace
 
-constexpr int OV_RATE_TABS = 48; /* doubling sizes: never reached */
-
 struct odevec_solver {
     int net;
     int64_t max_cells;
@@ -189,13 +188,7 @@ struct odevec_solver {
     size_t ord_temp_bytes;
     const int32_t* ord_cur; /* the last order computed, of ord_n cells */
     int64_t ord_n;
-    /* rate tables ([cells][reactions], networks with rate coefficients): the
-       last one is in use, of rate_cells cells; smaller ones before it stay
-       until odevec_close, since a captured graph may hold their address.
-       Each is at least twice the one before it */
-    int64_t rate_cells;
-    int rate_ntabs;
-    double* rate_tabs[OV_RATE_TABS];
+    ov::RateTables rates; /* of networks with rate coefficients */
 };
 /* d_queue words: [0] the solve's work counter, [1] cells that failed with
    FP32 factors, [2] the FP64 re-solve's work counter */
@@ -579,23 +572,9 @@ static cudaError_t rate_table(odevec_solver* s, ov::LaunchArgs& a, ov::launch_fn
     const int64_t nrea = g_nets[s->net].sizes[2];
     if (nrea <= 0 || a.ncells < OV_RATES_MIN_CELLS)
         return cudaSuccess;
-    if (s->rate_cells < a.ncells) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
-            s->rate_ntabs >= OV_RATE_TABS) {
-            cudaGetLastError();
-            return cudaSuccess;
-        }
-        const int64_t cells = a.ncells > 2 * s->rate_cells ? a.ncells : 2 * s->rate_cells;
-        double* tab = nullptr;
-        if (cudaMalloc(&tab, sizeof(double) * (size_t)nrea * (size_t)cells) != cudaSuccess) {
-            cudaGetLastError();
-            return cudaSuccess;
-        }
-        s->rate_tabs[s->rate_ntabs++] = tab;
-        s->rate_cells = cells;
-    }
-    a.rates = s->rate_tabs[s->rate_ntabs - 1];
+    a.rates = s->rates.get(a.ncells, nrea, st);
+    if (!a.rates)
+        return cudaSuccess;
     return fn(a, 1, 0, ov::STAGE_RATES, 0, 0, st);
 }
 
@@ -889,8 +868,7 @@ int32_t odevec_close(odevec_solver* s)
     cudaFree(s->ord_keys);
     cudaFree(s->ord_vals);
     cudaFree(s->ord_temp);
-    for (int i = 0; i < s->rate_ntabs; ++i)
-        cudaFree(s->rate_tabs[i]);
+    s->rates.close();
     cudaFree(s->d_y);
     cudaFree(s->d_t);
     cudaFree(s->d_dt);

@@ -80,3 +80,77 @@ int main()
     return 0;
 }
 """)
+
+
+FAKE_MEMORY = r"""
+#include "rate_tables.hpp"
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+static size_t g_room = 0;
+static bool g_capturing = false;
+static std::map<void*, size_t> g_live;
+extern "C" cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s)
+{
+    *s = g_capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaGetLastError() { return cudaSuccess; }
+extern "C" cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode*) { return cudaSuccess; }
+extern "C" cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { *f = g_room; *t = g_room; return cudaSuccess; }
+extern "C" cudaError_t cudaMalloc(void** p, size_t n)
+{
+    if (g_capturing || n > g_room)
+        return cudaErrorMemoryAllocation;
+    *p = std::malloc(1);
+    g_live[*p] = n;
+    g_room -= n;
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaFree(void* p)
+{
+    if (g_live.count(p) != 1)
+        std::abort();
+    g_room += g_live[p];
+    g_live.erase(p);
+    std::free(p);
+    return cudaSuccess;
+}
+static size_t live() { size_t n = 0; for (auto& e : g_live) n += e.second; return n; }
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
+"""
+
+
+def test_rate_tables_memory(tmp_path):
+    """A solver whose cell count grows holds one table; a table in a graph stays
+    where it is; none is taken where it would leave less than half of the free
+    memory; what no graph holds can be given back."""
+    _run(tmp_path, FAKE_MEMORY + r"""
+int main()
+{
+    const int64_t nrea = 38, B = 8 * nrea;
+    g_room = 12000 * B; /* half of what the table of at most 2,248 cells leaves holds twice as much */
+    ov::RateTables r = {};
+    double* a = r.get(1000, nrea, 0);
+    CHECK(a && live() == (size_t)(1000 * B));
+    CHECK(r.get(700, nrea, 0) == a && r.get(1000, nrea, 0) == a);
+    for (int64_t n = 1001; n < 2000; ++n) { /* one table, at most an eighth too large */
+        CHECK(r.get(n, nrea, 0) && live() >= (size_t)(n * B) && live() <= (size_t)((n + n / 8) * B));
+    }
+    g_capturing = true;
+    double* g = r.get(1500, nrea, 0); /* now in a graph */
+    const size_t held = live();
+    CHECK(g && r.get(9000, nrea, 0) == nullptr && live() == held);
+    g_capturing = false;
+    CHECK(r.get(1500, nrea, 0) == g && !r.drop());
+    double* b = r.get(3000, nrea, 0);
+    CHECK(b && b != g && live() >= 3 * held); /* at least twice the one before */
+    CHECK(r.drop() && live() == held && !r.drop());
+    CHECK(r.get(9000, nrea, 0) == nullptr && live() == held); /* more than half of what is free */
+    CHECK(r.get(3000, nrea, 0) && r.get(1500, nrea, 0));
+    r.close();
+    CHECK(live() == 0 && r.n == 0 && r.get(1000, nrea, 0));
+    r.close();
+    return 0;
+}
+""")
