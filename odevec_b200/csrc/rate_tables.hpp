@@ -20,6 +20,15 @@
 
 namespace ov {
 
+/* Another thread or stream may be capturing in the default (global) mode, in
+   which an allocation anywhere fails and spoils the capture; the allocations
+   here belong to no graph */
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 struct RateTables {
     static constexpr int MAX = 48; /* doubling sizes: never reached */
     int n;
@@ -48,6 +57,7 @@ struct RateTables {
             if (n == MAX)
                 return nullptr;
             const size_t bytes = sizeof(double) * (size_t)nrea * (size_t)want;
+            RelaxedCapture relaxed;
             size_t room = 0, total = 0;
             void* p = nullptr;
             if (cudaMemGetInfo(&room, &total) != cudaSuccess || bytes > room / 2 ||
@@ -69,6 +79,7 @@ struct RateTables {
     {
         if (n == 0 || captured)
             return false;
+        RelaxedCapture relaxed;
         cudaFree(tab[--n]); /* waits for the kernels that use it */
         captured = n > 0;
         return true;

@@ -381,3 +381,29 @@ def test_continuation_of_a_replayed_solve(gpu_lib, oracle, na, nb):
         S.set_yield(ode, None)
     finally:
         S.CloseOdevec(ode)
+
+
+def test_solve_beside_a_capture(gpu_lib, oracle):
+    """A solve on one stream, which allocates its rate table, while another
+    stream is being captured in the global mode: both come out whole."""
+    import torch
+    S = gpu_lib
+    wl = W.primordial(ncells=5000, seed=33)
+    wl.t_stop[:] = 1e6
+    ode = _solver(S, wl)
+    try:
+        y, t, d, ts = (torch.tensor(v, device="cuda") for v in (wl.y, wl.t0, wl.dt0, wl.t_stop))
+        st = torch.zeros(wl.ncells, dtype=torch.int32, device="cuda")
+        x = torch.ones(64, device="cuda")
+        other = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            x.add_(1.0)
+            S.SolveODERange(ode, 0, wl.ncells, t, d, ts, y, st, stream=other)
+        g.replay()
+        torch.cuda.synchronize()
+        assert float(x[0]) == 2.0
+        _same([v.cpu().numpy() for v in (y, t, d, st)], _oracle(oracle, wl)[:4])
+    finally:
+        S.CloseOdevec(ode)
