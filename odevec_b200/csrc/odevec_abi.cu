@@ -527,14 +527,14 @@ static int32_t visit_order(odevec_solver* s, int64_t ncells, const double* t, co
         s->ord_cur = nullptr;
         s->ord_n = 0;
         const size_t n = (size_t)ncells;
-        err = cudaMalloc(&s->ord_keys, 2 * n * sizeof(uint16_t));
-        if (err == cudaSuccess) err = cudaMalloc(&s->ord_vals, 2 * n * sizeof(int32_t));
+        err = s->rates.alloc(&s->ord_keys, 2 * n * sizeof(uint16_t));
+        if (err == cudaSuccess) err = s->rates.alloc(&s->ord_vals, 2 * n * sizeof(int32_t));
         if (err == cudaSuccess) {
             cub::DoubleBuffer<uint16_t> kb(s->ord_keys, s->ord_keys + n);
             cub::DoubleBuffer<int32_t> vb(s->ord_vals, s->ord_vals + n);
             err = cub::DeviceRadixSort::SortPairsDescending(nullptr, s->ord_temp_bytes, kb, vb, (int)n, 0, 16, st);
         }
-        if (err == cudaSuccess) err = cudaMalloc(&s->ord_temp, s->ord_temp_bytes);
+        if (err == cudaSuccess) err = s->rates.alloc(&s->ord_temp, s->ord_temp_bytes);
         if (err != cudaSuccess)
             return fail(OV_API_ENOMEM, "odevec_solve: visit order buffers: %s", cudaGetErrorString(err));
         s->ord_cells = ncells;
@@ -667,11 +667,11 @@ static int32_t solve_impl(odevec_solver* s, int64_t ncells, int64_t stride, doub
             s->fb_y = nullptr; s->fb_t = nullptr; s->fb_dt = nullptr; s->fb_status = nullptr; s->fb_mask = nullptr;
             s->fb_cells = 0;
             const size_t n = (size_t)ncells;
-            err = cudaMalloc(&s->fb_y, sizeof(double) * n * neq);
-            if (err == cudaSuccess) err = cudaMalloc(&s->fb_t, sizeof(double) * n);
-            if (err == cudaSuccess) err = cudaMalloc(&s->fb_dt, sizeof(double) * n);
-            if (err == cudaSuccess) err = cudaMalloc(&s->fb_status, sizeof(int32_t) * n);
-            if (err == cudaSuccess) err = cudaMalloc(&s->fb_mask, n);
+            err = s->rates.alloc(&s->fb_y, sizeof(double) * n * neq);
+            if (err == cudaSuccess) err = s->rates.alloc(&s->fb_t, sizeof(double) * n);
+            if (err == cudaSuccess) err = s->rates.alloc(&s->fb_dt, sizeof(double) * n);
+            if (err == cudaSuccess) err = s->rates.alloc(&s->fb_status, sizeof(int32_t) * n);
+            if (err == cudaSuccess) err = s->rates.alloc(&s->fb_mask, n);
             if (err != cudaSuccess)
                 return fail(OV_API_ENOMEM, "odevec_solve: escalation buffers: %s", cudaGetErrorString(err));
             s->fb_cells = ncells;
@@ -1164,11 +1164,22 @@ extern "C" int32_t odevec_solve_many(const odevec_job* jobs, int32_t njobs, void
         if (err != cudaSuccess)
             return fail(OV_API_ECUDA, "odevec_solve_many: %s", cudaGetErrorString(err));
         /* each job's cells longest span first, as odevec_solve visits them */
-        const int32_t rc = visit_order(J.solver, J.ncells, J.t, J.t_stop, st, &a.order);
+        int32_t rc = visit_order(J.solver, J.ncells, J.t, J.t_stop, st, &a.order);
+        if (rc == OV_API_ENOMEM) {
+            bool freed = false;
+            for (int k = 0; k < nlive; ++k)
+                freed = jobs[live[k]].solver->rates.drop() || freed;
+            if (freed)
+                rc = visit_order(J.solver, J.ncells, J.t, J.t_stop, st, &a.order);
+        }
         if (rc)
             return rc;
-        const NetEntry& e = g_nets[J.solver->net];
-        err = rate_table(J.solver, a, prec == OV_PREC_FP64 ? e.exact : e.fma, st);
+    }
+    /* the tables last: they are optional, the buffers above are not */
+    for (int q = 0; q < nlive; ++q) {
+        odevec_solver* s = jobs[live[q]].solver;
+        const NetEntry& e = g_nets[s->net];
+        const cudaError_t err = rate_table(s, P.job[q], prec == OV_PREC_FP64 ? e.exact : e.fma, st);
         if (err != cudaSuccess)
             return fail(OV_API_ECUDA, "odevec_solve_many: %s", cudaGetErrorString(err));
     }

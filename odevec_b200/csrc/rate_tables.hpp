@@ -85,6 +85,19 @@ struct RateTables {
         return true;
     }
 
+    /* cudaMalloc for a buffer that a solve cannot do without: where there is no
+       room, the newest table gives way */
+    template <class T>
+    cudaError_t alloc(T** p, size_t bytes)
+    {
+        cudaError_t e = cudaMalloc((void**)p, bytes);
+        if (e == cudaErrorMemoryAllocation && drop())
+            e = cudaMalloc((void**)p, bytes);
+        if (e != cudaSuccess)
+            cudaGetLastError(); /* the caller returns it */
+        return e;
+    }
+
     void close()
     {
         while (n > 0)

@@ -154,3 +154,29 @@ int main()
     return 0;
 }
 """)
+
+
+def test_rate_tables_give_way(tmp_path):
+    """A buffer that a solve needs takes the place of the newest table where there
+    is no room for both, but not of a table that a graph may hold."""
+    _run(tmp_path, FAKE_MEMORY + r"""
+int main()
+{
+    const int64_t nrea = 38, B = 8 * nrea;
+    g_room = 2000 * B;
+    ov::RateTables r = {};
+    double* p = nullptr;
+    CHECK(r.get(1000, nrea, 0) && r.alloc(&p, 900 * B) == cudaSuccess && r.n == 1);
+    cudaFree(p);
+    CHECK(r.alloc(&p, 1500 * B) == cudaSuccess && r.n == 0 && live() == (size_t)(1500 * B));
+    CHECK(r.get(1000, nrea, 0) == nullptr); /* the solve then goes without */
+    cudaFree(p);
+    CHECK(r.get(1000, nrea, 0));
+    g_capturing = true;
+    CHECK(r.get(1000, nrea, 0));
+    g_capturing = false;
+    CHECK(r.alloc(&p, 1500 * B) == cudaErrorMemoryAllocation && r.n == 1);
+    r.close();
+    return 0;
+}
+""")
