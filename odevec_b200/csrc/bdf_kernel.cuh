@@ -1685,13 +1685,8 @@ cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream
     const bool chosen = block > 0 || grid > 0; /* the caller fixes the shape */
     if (Cfg::SHM || block <= 0 || block > Cfg::BS)
         block = Cfg::BS;
-    static Residency residency;
-    int sms = 0, resident = 0;
+    int sms = 0;
     cudaError_t err = device_sms(&sms);
-    if (err == cudaSuccess)
-        err = allow_smem((const void*)kern, smem);
-    if (err == cudaSuccess)
-        err = resident_blocks(residency, (const void*)kern, block, smem, &resident);
     if (err != cudaSuccess)
         return err;
     LaunchArgs b = a;
@@ -1716,6 +1711,11 @@ cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream
         if (!chosen && a.ncells <= lanes * per_lane)
             return launch<Net, G, LUT, SPREAD_STAGE>(a, 0, 0, stream);
     }
+    /* only now, since a question about a kernel loads it: a process of small
+       solves loads the one kernel that it runs */
+    err = allow_smem((const void*)kern, smem);
+    if (err != cudaSuccess)
+        return err;
     if (Net::ND <= 32 && !chosen && a.ncells <= (int64_t)sms * SPREAD_WARPS * 32) {
         /* Few cells: over all SMs, at most one warp per scheduler and only as
            many lanes per warp as that takes.  The time is that of the longest
@@ -1743,7 +1743,10 @@ cudaError_t launch(const LaunchArgs& a, int block, int grid, cudaStream_t stream
         if (grid < 1)
             grid = 1;
     } else if (grid <= 0) {
-        grid = resident;
+        static Residency residency;
+        err = resident_blocks(residency, (const void*)kern, block, smem, &grid);
+        if (err != cudaSuccess)
+            return err;
         const int64_t warps_needed = (a.ncells + 31) / 32;
         const int64_t blocks_needed = (warps_needed * 32 + block - 1) / block;
         if (blocks_needed < grid)

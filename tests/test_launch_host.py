@@ -180,3 +180,14 @@ int main()
     return 0;
 }
 """)
+
+
+def test_launch_loads_one_kernel():
+    """The launcher hands a solve of few cells to the other shape's kernel before
+    it asks the runtime anything about its own, which would load it."""
+    text = open(os.path.join(CSRC, "bdf_kernel.cuh")).read()
+    body = text[text.index("cudaError_t launch(const LaunchArgs& a, int block, int grid"):]
+    body = body[:body.index("kern<<<")]
+    other = body.index("return launch<Net, G, LUT, SPREAD_STAGE>")
+    for question in ("allow_smem(", "resident_blocks("):
+        assert body.count(question) == 1 and body.index(question) > other
