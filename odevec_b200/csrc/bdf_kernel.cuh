@@ -1991,7 +1991,9 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
                 OV_STAGE_CASE(NET, double, 16)                                               \
                 if constexpr (blk_ok<NET, double>()) {                                       \
                     if constexpr (BLK_SPLIT && y_fits<NET, 256>()) {                         \
-                        if (a.ncells >= BLK_SPLIT_CELLS) {                                   \
+                        int sms = 0;                                                         \
+                        if (stage == 18 && device_sms(&sms) == cudaSuccess &&                \
+                            a.ncells >= blk_split_cells(sms)) {                              \
                             OV_STAGE_CASE(NET, double, 18)                                   \
                         }                                                                    \
                     }                                                                        \

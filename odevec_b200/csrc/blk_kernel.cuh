@@ -55,13 +55,16 @@ constexpr bool BLK_SPLIT = true;
 #endif
 
 /* Without contraction a thread per cell (staging 18's other form) is the faster
-   one from two cells per lane on, 256 lanes on each of 148 SMs: its divisions
-   run for 32 cells beside seven other warps' work, here in one warp while the
-   others wait.  SYN64 FP64, thread per cell / block per 32 cells: 37,888
-   cells 290 / 302 ms, 65,536 cells 526 / 521, 75,776 cells 560 / 599,
-   262,144 cells 1,810 / 2,060; 3,001 cells 157 / 38.  (With contraction
-   262,144 cells take 1,624 ms here against 1,910, FP32-LU 944 against 1,530.) */
-constexpr int64_t BLK_SPLIT_CELLS = 2 * 148 * 256;
+   one from two cells per lane on, in blocks of 256: its divisions run for 32
+   cells beside seven other warps' work, here in one warp while the others
+   wait.  SYN64 FP64 on 148 SMs, thread per cell / block per 32 cells: 3,001
+   cells 157 / 38 ms, 37,888 cells 290 / 302, 65,536 cells 526 / 521, 75,776
+   cells (the line) 560 / 599, 262,144 cells 1,810 / 2,060.  The one size in
+   between where a thread per cell is ahead as well, by 4 %, is that of one cell
+   for every lane.  (With contraction 262,144 cells take 1,624 ms here against
+   1,910, FP32-LU 944 against 1,530.) */
+constexpr int BLK_SPLIT_THREADS = 256;
+constexpr int64_t blk_split_cells(int sms) { return (int64_t)2 * sms * BLK_SPLIT_THREADS; }
 
 template <class Net, class LUT>
 struct BlkLayout {

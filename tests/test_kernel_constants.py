@@ -91,3 +91,12 @@ def test_quotient_iteration(kind):
         q = fma(fma(-q, d, x), r, q)
         q = fma(fma(-q, d, x), r, q)
         assert q == x / d
+
+
+def test_no_rule_for_one_chip():
+    """The launch rules take the SM count from the device."""
+    csrc = os.path.dirname(CUH)
+    for name in os.listdir(csrc):
+        if name.endswith((".cuh", ".cu", ".h", ".hpp")):
+            code = re.sub(r"/\*.*?\*/|//[^\n]*", "", open(os.path.join(csrc, name)).read(), flags=re.S)
+            assert not re.search(r"\b148\b", code), name
