@@ -1827,8 +1827,6 @@ struct MultiJob {
     }
     __device__ __forceinline__ static void run(const LaunchArgs& A)
     {
-        /* both begin with a barrier, so no warp touches the shared memory of
-           this job while another still works on the one before */
         if constexpr (BLOCK)
             blk_run<Net, LUT>(A);
         else
@@ -1872,6 +1870,11 @@ __global__ void __launch_bounds__(MULTI_BS, 1) bdf_multi_kernel(const __grid_con
     for (int k = 0; k < P.njobs; ++k) {
         const int j = (first + k) % P.njobs;
         MultiDispatch<LUT, Nets...>::run(P.net[j], P.job[j]);
+        /* a warp that leaves a job's loop first must not set up the lockstep
+           words of the next job, if of the same network, while others use them
+           (two jobs of 65,536 PRIMORDIAL cells, FP32-LU: 166-191 ms, 20 so; in
+           front of the set-up the barrier costs a third of the speed) */
+        __syncthreads();
     }
 }
 

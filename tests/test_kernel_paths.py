@@ -407,3 +407,42 @@ def test_solve_beside_a_capture(gpu_lib, oracle):
         _same([v.cpu().numpy() for v in (y, t, d, st)], _oracle(oracle, wl)[:4])
     finally:
         S.CloseOdevec(ode)
+
+
+def test_multi_jobs_of_one_network(gpu_lib):
+    """Two jobs of one network in one launch keep the bits of one job of all the
+    cells, and its time: a warp that has left the first job's loop must not
+    take the lockstep words from those that have not (each of their trips then
+    waits out its limit, ten times the time)."""
+    import torch
+    from odevec_b200.multi import SolveMany
+    S = gpu_lib
+    n = 60000
+    wl = W.primordial(ncells=n, seed=14)
+    got, ms = [], []
+    for cut in (n, n // 2):
+        odes = [_solver(S, wl) for _ in range(n // cut)]
+        try:
+            best = None
+            for _ in range(3):
+                jobs = []
+                for k, ode in enumerate(odes):
+                    part = slice(k * cut, (k + 1) * cut)
+                    jobs.append((ode, *[torch.tensor(a[..., part], device="cuda")
+                                        for a in (wl.t0, wl.dt0, wl.t_stop, wl.y)]))
+                many = SolveMany(jobs, fused=True)
+                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                torch.cuda.synchronize()
+                e0.record()
+                many.run()
+                e1.record()
+                torch.cuda.synchronize()
+                best = e0.elapsed_time(e1) if best is None else min(best, e0.elapsed_time(e1))
+            got.append([torch.cat([j[k] for j in jobs], dim=-1).cpu().numpy() for k in (1, 2, 4)])
+            ms.append(best)
+        finally:
+            for ode in odes:
+                S.CloseOdevec(ode)
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+    assert ms[1] < 3.0 * ms[0], ms
