@@ -1248,7 +1248,7 @@ __device__ __forceinline__ void bdf_run(const LaunchArgs& A)
             soft.gen = 0u;
             soft.active = blockDim.x / 32u;
         }
-        __syncthreads(); /* once, at entry, with every thread converged */
+        __syncthreads(); /* at entry, with every thread converged */
     }
 
     /* A continued solve is a short one (a hydro step: some twelve steps a
@@ -1814,54 +1814,68 @@ namespace OV_MODE_NS {
    16,384 ROBER, 65,536 PRIMORDIAL and 4,096 SYN64 cells, FP32-LU: 190 ms with
    every network on one 384-thread block per SM and shares by cells alone,
    46 ms so. */
-template <class Net, class LUT>
+template <class Net, class LUT, bool MANY>
 struct MultiJob {
     static constexpr int STAGE = hist_fits<Net, 256>() ? 9 : 15;
     static constexpr bool BLOCK = blk_ok<Net, LUT>();
+    /* a kernel for launches with many cells of it: a thread per cell for those
+       (blk_split_cells) */
+    static constexpr bool SPLIT = MANY && BLOCK && BLK_SPLIT && y_fits<Net, BLK_SPLIT_THREADS>();
     static constexpr size_t smem()
     {
-        if constexpr (BLOCK)
+        if constexpr (SPLIT) {
+            constexpr size_t a = BlkLayout<Net, LUT>::smem_bytes;
+            constexpr size_t b = Staging<Net, LUT, StageCfg<18>::SHM, StageCfg<18>::BS>::smem_bytes;
+            return a > b ? a : b;
+        } else if constexpr (BLOCK) {
             return BlkLayout<Net, LUT>::smem_bytes;
-        else
+        } else {
             return Staging<Net, LUT, StageCfg<STAGE>::SHM, StageCfg<STAGE>::BS>::smem_bytes;
+        }
     }
-    __device__ __forceinline__ static void run(const LaunchArgs& A)
+    __device__ __forceinline__ static void run(const LaunchArgs& A, bool many)
     {
-        if constexpr (BLOCK)
+        if constexpr (SPLIT) {
+            if (many)
+                bdf_run<Net, 1, LUT, 18>(A);
+            else
+                blk_run<Net, LUT>(A);
+        } else if constexpr (BLOCK) {
             blk_run<Net, LUT>(A);
-        else
+        } else {
             bdf_run<Net, 1, LUT, STAGE>(A);
+        }
     }
 };
 constexpr int MULTI_BS = 256;
 static_assert(32 * BLK_WARPS == MULTI_BS && StageCfg<9>::BS == MULTI_BS && StageCfg<15>::BS == MULTI_BS &&
-                  StageCfg<9>::SOFT && StageCfg<15>::SOFT,
+                  StageCfg<18>::BS == MULTI_BS && StageCfg<9>::SOFT && StageCfg<15>::SOFT && StageCfg<18>::SOFT,
               "the jobs of a multi-network launch share one block shape and start with a barrier");
 
-template <class LUT, class... Nets>
+template <class LUT, bool MANY, class... Nets>
 constexpr size_t multi_smem_bytes()
 {
     size_t m = 0;
-    ((m = MultiJob<Nets, LUT>::smem() > m ? MultiJob<Nets, LUT>::smem() : m), ...);
+    ((m = MultiJob<Nets, LUT, MANY>::smem() > m ? MultiJob<Nets, LUT, MANY>::smem() : m), ...);
     return m;
 }
 
-template <class LUT, class... Nets>
+template <class LUT, bool MANY, class... Nets>
 struct MultiDispatch {
-    __device__ __forceinline__ static void run(int, const LaunchArgs&) {}
+    __device__ __forceinline__ static void run(int, const LaunchArgs&, bool) {}
 };
-template <class LUT, class Net0, class... Rest>
-struct MultiDispatch<LUT, Net0, Rest...> {
-    __device__ __forceinline__ static void run(int idx, const LaunchArgs& A)
+template <class LUT, bool MANY, class Net0, class... Rest>
+struct MultiDispatch<LUT, MANY, Net0, Rest...> {
+    __device__ __forceinline__ static void run(int idx, const LaunchArgs& A, bool many)
     {
         if (idx == 0)
-            MultiJob<Net0, LUT>::run(A);
+            MultiJob<Net0, LUT, MANY>::run(A, many);
         else
-            MultiDispatch<LUT, Rest...>::run(idx - 1, A);
+            MultiDispatch<LUT, MANY, Rest...>::run(idx - 1, A, many);
     }
 };
 
-template <class LUT, class... Nets>
+template <class LUT, bool MANY, class... Nets>
 __global__ void __launch_bounds__(MULTI_BS, 1) bdf_multi_kernel(const __grid_constant__ MultiArgs P)
 {
     int first = 0;
@@ -1869,7 +1883,7 @@ __global__ void __launch_bounds__(MULTI_BS, 1) bdf_multi_kernel(const __grid_con
         ++first;
     for (int k = 0; k < P.njobs; ++k) {
         const int j = (first + k) % P.njobs;
-        MultiDispatch<LUT, Nets...>::run(P.net[j], P.job[j]);
+        MultiDispatch<LUT, MANY, Nets...>::run(P.net[j], P.job[j], P.many[j] != 0);
         /* a warp that leaves a job's loop first must not set up the lockstep
            words of the next job, if of the same network, while others use them
            (two jobs of 65,536 PRIMORDIAL cells, FP32-LU: 166-191 ms, 20 so; in
@@ -1880,11 +1894,11 @@ __global__ void __launch_bounds__(MULTI_BS, 1) bdf_multi_kernel(const __grid_con
 
 /* Launches the multi-network kernel on P (block ranges filled in here in
    proportion to the jobs' work, at least one block per job). */
-template <class LUT, class... Nets>
-cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
+template <class LUT, bool MANY, class... Nets>
+cudaError_t launch_multi_kernel(MultiArgs& P, cudaStream_t stream)
 {
-    auto kern = bdf_multi_kernel<LUT, Nets...>;
-    constexpr size_t smem = multi_smem_bytes<LUT, Nets...>();
+    auto kern = bdf_multi_kernel<LUT, MANY, Nets...>;
+    constexpr size_t smem = multi_smem_bytes<LUT, MANY, Nets...>();
     static_assert(smem <= 226 * 1024, "the set's largest state vectors exceed a block's shared memory");
     static Residency residency;
     int resident = 0;
@@ -1894,7 +1908,7 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
     if (err != cudaSuccess)
         return err;
     const int nnz[] = {Nets::NNZ...};
-    const bool block[] = {MultiJob<Nets, LUT>::BLOCK...};
+    const bool block[] = {MultiJob<Nets, LUT, MANY>::BLOCK...};
     /* Blocks of each job: first a block per 32 cells for the large networks
        (all but one per other job at most), whose cells take longest from
        start to end; the rest in proportion to cells times LU entries, an
@@ -1928,6 +1942,31 @@ cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
     P.block_start[P.njobs] = start;
     kern<<<start, MULTI_BS, smem, stream>>>(P);
     return cudaGetLastError();
+}
+
+/* The thread-per-cell body of a large network is in a kernel of its own, for
+   the launches that use it: beside it the compiler gives the other networks'
+   bodies less (131,072 PRIMORDIAL cells, FP64: 32.0 ms without, 39.3 with).
+   65,536 ROBER, 262,144 PRIMORDIAL and 262,144 SYN64 cells, FP64: 2,351 ms
+   with SYN64 in the block kernel, 2,036 so. */
+template <class LUT, class... Nets>
+cudaError_t launch_multi(MultiArgs& P, cudaStream_t stream)
+{
+    if constexpr ((MultiJob<Nets, LUT, true>::SPLIT || ...)) {
+        const bool split[] = {MultiJob<Nets, LUT, true>::SPLIT...};
+        int sms = 0;
+        const cudaError_t err = device_sms(&sms);
+        if (err != cudaSuccess)
+            return err;
+        bool any = false;
+        for (int j = 0; j < P.njobs; ++j) {
+            P.many[j] = split[P.net[j]] && P.job[j].ncells >= blk_split_cells(sms);
+            any = any || P.many[j];
+        }
+        if (any)
+            return launch_multi_kernel<LUT, true, Nets...>(P, stream);
+    }
+    return launch_multi_kernel<LUT, false, Nets...>(P, stream);
 }
 
 }  // namespace OV_MODE_NS

@@ -82,6 +82,7 @@ struct MultiArgs {
     LaunchArgs job[MULTI_MAX_JOBS];
     int32_t net[MULTI_MAX_JOBS];
     int32_t block_start[MULTI_MAX_JOBS + 1];
+    int32_t many[MULTI_MAX_JOBS]; /* a large network's job has many cells: a thread per cell where both forms exist */
     int32_t njobs;
 };
 typedef cudaError_t (*multi_fn)(MultiArgs& P, int lu, cudaStream_t stream);

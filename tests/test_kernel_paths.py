@@ -446,3 +446,34 @@ def test_multi_jobs_of_one_network(gpu_lib):
     for a, b in zip(*got):
         assert np.array_equal(a, b)
     assert ms[1] < 3.0 * ms[0], ms
+
+
+@pytest.mark.parametrize("n", [75775, 75776])
+def test_multi_block_limit(gpu_lib, n):
+    """The large network's cells in a launch of several networks, in FP64 below
+    and from the line on where they run one to a thread: the bits of separate
+    solves."""
+    import torch
+    from odevec_b200.multi import SolveMany
+    S = gpu_lib
+    got = []
+    for fused in (True, False):
+        wls = [W.rober(33, seed=2), W.syn64(n, seed=12), W.primordial(5000, seed=2)]
+        wls[1].t_stop[:] = 1e-6
+        odes, jobs = [], []
+        for wl in wls:
+            odes.append(_solver(S, wl, nvector=1))
+            jobs.append((odes[-1], *[torch.tensor(a, device="cuda") for a in (wl.t0, wl.dt0, wl.t_stop, wl.y)]))
+        try:
+            if fused:
+                SolveMany(jobs, fused=True).run()
+            else:
+                for ode, t, d, ts, y in jobs:
+                    S.SolveODE(ode, t, d, ts, y)
+            torch.cuda.synchronize()
+            got.append([a.cpu().numpy() for ode, t, d, ts, y in jobs for a in (y, t, d, ode.status)])
+        finally:
+            for ode in odes:
+                S.CloseOdevec(ode)
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
