@@ -110,12 +110,14 @@ typedef struct odevec_opts {
        memory, 20 = as 3 with the state vector in shared memory (18-20:
        networks above 32 solver species; 18 is one block of eight warps per
        32 cells, which share a cell's species, for constant-coefficient
-       networks of up to 64 species with the symbolic Jacobian, and for solves
-       in FP64 without contraction below 75,776 cells); 21 = as 3 with the history in
-       shared memory and each block in soft lockstep (up to 12 solver
-       species) (2-21: per-cell control only).  In 2-6 and 8-16 idle lanes take new cells on every
-       16th trip of the cell loop (17: every 32nd), so cells are set up
-       several at a time (in 8-12 and 15-17 in all warps of a block at
+       networks of up to 64 species with the symbolic Jacobian; in FP64 without
+       contraction below two cells for each of 256 lanes per SM, 75,776 cells
+       on 148 SMs); 21 = as 3 with the history in shared memory and each block
+       in soft lockstep (up to 12 solver species) (2-21: per-cell control
+       only).  In 2-6, 8-16 and 19-21 idle lanes take new cells on every 16th
+       trip of the cell loop (17: every 32nd; a solve with resume = 1: every
+       4th; 18: every 4th in its block form, else every 16th), so cells are set
+       up several at a time (in 8-12, 15-19 and 21 in all warps of a block at
        once); staging 1 refills on every trip.  block_threads (a multiple of 32 up to
        the block of the staging) and grid_blocks: 0 = automatic (persistent
        grid filling every SM) */
@@ -157,7 +159,19 @@ int32_t odevec_set_options(odevec_solver* s, const odevec_opts* opts);
    mask (nullable): cells with mask 0 are left untouched except t = t_stop.
    status, stats: nullable outputs.  With per-cell control and at least
    32,768 cells the cells are visited longest t_stop - t first (a device
-   sort on the stream); results do not depend on the order. */
+   sort on the stream); results do not depend on the order.
+
+   Device memory: besides odevec_init's, the solver allocates, in the first
+   call that needs it or needs more of it, and keeps until odevec_close: the
+   order's buffers (from 32,768 cells on, 12 bytes per cell and the sort's),
+   the inputs of cells that may be solved again (OV_PREC_FP32_LU with
+   escalation, 8 neq + 21 bytes per cell), and, for networks with rate
+   coefficients, from 4,096 cells on a table of them (8 nrea bytes per cell, 304
+   for PRIMORDIAL).  The table is optional: it is taken only where it leaves
+   half of the free memory, gives way to the other buffers, and without it
+   results are the same.  A captured call uses the buffers as they are: make
+   one eager call of the largest count first, and no larger one while the graph
+   lives (a table in a graph stays until odevec_close). */
 int32_t odevec_solve(odevec_solver* s, int64_t ncells, double* y, double* t, double* dt,
                      const double* t_stop, const uint8_t* mask, int32_t* status, int32_t* stats,
                      void* stream);
@@ -223,8 +237,8 @@ int32_t odevec_solve_range(odevec_solver* s, int64_t ncells, int64_t stride, dou
    odevec_cells_started(s, stream, &n) synchronises `stream` and reads how
    many cells the solve has started (n >= ncells: all of them; n may exceed
    ncells).  odevec_solve_continue takes odevec_solve_range's arguments
-   (the same arrays as the solve it continues) and starts the cells not yet
-   started.  With OV_PREC_FP32_LU the escalation of failed cells runs after
+   (the same arrays as the solve it continues, which must be the last that ran
+   on s, as a call or as a replayed graph) and starts the cells not yet started.  With OV_PREC_FP32_LU the escalation of failed cells runs after
    the launch that completes the solve.  Results are those of one
    uninterrupted solve: every cell runs once, on its own. */
 int32_t odevec_set_yield(odevec_solver* s, const int32_t* flag);
@@ -260,10 +274,10 @@ const char* odevec_last_error(void);
    across jobs), cells and arrays.  All jobs must use the same precision
    form and per-cell control (group_size 1); the launch uses one compiled
    multi-network kernel whose set of variants holds every job's network
-   (OV_API_EUNSUPPORTED if none does).  The kernel gives each job a share of
-   the blocks in proportion to its cells, and a block whose job has no cells
-   left takes cells of the others, so the networks share the device for the
-   whole launch; each job's cells are visited longest t_stop - t first, as
+   (OV_API_EUNSUPPORTED if none does).  A large network's cells get their
+   blocks first, the other jobs share the rest in proportion to their work (cells
+   times LU entries), and a block whose job has no cells left takes cells of
+   the others, so the networks share the device for the whole launch; each job's cells are visited longest t_stop - t first, as
    in odevec_solve.  Failed FP32-LU cells are not solved again (see
    no_escalation).  Asynchronous on stream. */
 #define OV_MULTI_MAX_JOBS 8

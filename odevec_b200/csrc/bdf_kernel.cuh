@@ -3,8 +3,8 @@
  * One thread integrates one cell.  A warp is either 32 independent cells
  * (G = 1: per-cell time, step, order and Jacobian decisions) or one lockstep
  * group of 32 cells that share them through max-norms over the warp
- * (G = 32: the reference's semantics with nvector = 32, reductions with
- * __shfl_xor_sync).  The grid is persistent: idle lanes take the next cells
+ * (G = 32: the reference's semantics with nvector = 32, with warp
+ * reductions).  The grid is persistent: idle lanes take the next cells
  * from a global counter (warp-aggregated atomicAdd), so a warp keeps its
  * lanes busy while cells of very different stiffness finish at different
  * times.
@@ -34,9 +34,10 @@
  *
  * Per-cell state: en, en_old, error weights, the state and the packed LU in
  * thread-local arrays with compile-time indices (the LU in shared memory for
- * stagings 2, 5 and 11); the Nordsieck history y_NS(0:5), which loops over
- * the runtime order index, in a thread-local array or, for stagings 2, 5 and
- * 9-11, in shared memory laid out [entry][lane].  The staging (StageCfg) also
+ * stagings 2, 5, 11 and 22, the launcher's own); the Nordsieck history
+ * y_NS(0:5), which loops over the runtime order index, in a thread-local array
+ * or, for stagings 2, 5, 9-12, 17, 21 and 22, in shared memory laid out
+ * [entry][lane]; up to four species it stays in registers elsewhere.  The staging (StageCfg) also
  * fixes the block size, the blocks per SM, whether the block's warps run in
  * soft lockstep and how often idle lanes take new cells.
  *
@@ -383,7 +384,10 @@ __device__ __forceinline__ void soft_leave(SoftSync* s, int lane)
 /* An FP64 LU with the correctly rounded reciprocals of its pivots beside it.
    A division by a pivot is then five dependent fused multiply-adds without a
    branch: the quotient from the reciprocal, corrected twice with its exact
-   residual, which rounds correctly (P. Markstein, IBM J. Res. Dev. 34, 1990).
+   residual, which rounds correctly (P. Markstein, IBM J. Res. Dev. 34, 1990)
+   up to the sign of zero: -0 by a positive pivot gives +0.  No result sees it:
+   in the factors and solves a zero only adds and multiplies, and a correction
+   is added to a sum that starts at +0.
    Operands for which that is not certain (far exponents, infinities, NaN, an
    all-ones significand) are recorded in bad, and the caller repeats the work
    with IEEE divisions.  The generated factorisation and solves pick these
@@ -1808,12 +1812,14 @@ namespace OV_MODE_NS {
 /* One block of 256 threads per SM with all the registers of a thread.  A job
    runs as its network runs best alone: a large network as one block per 32
    cells (blk_kernel.cuh), another as staging 9 (soft lockstep, the history in
-   shared memory) or, where a history does not fit, staging 15.  The blocks are
+   shared memory) or, where a history does not fit, staging 15.  A large
+   network's cells, which take longest, get their blocks first, the rest are
    shared out in proportion to cells times LU entries, an estimate of the
    jobs' work; a block whose job has no cells left takes cells of the others.
-   16,384 ROBER, 65,536 PRIMORDIAL and 4,096 SYN64 cells, FP32-LU: 190 ms with
-   every network on one 384-thread block per SM and shares by cells alone,
-   46 ms so. */
+   16,384 ROBER, 65,536 PRIMORDIAL and 4,096 SYN64 cells, FP32-LU / FP64: 196 /
+   254 ms with every network on one 384-thread block per SM and shares by cells
+   alone, 40 / 60 ms so (46 with FP32-LU before the large network came first);
+   65,536, 262,144 and 16,384 cells: 303 / 415 and 131 / 213 ms. */
 template <class Net, class LUT, bool MANY>
 struct MultiJob {
     static constexpr int STAGE = hist_fits<Net, 256>() ? 9 : 15;

@@ -21,13 +21,16 @@
  * as in bdf_kernel.cuh, whose phases (Phase, SsMode) and network code this
  * kernel shares; results equal its results bit for bit.
  *
- * Bound by instruction fetch: a trip walks through some 200 KB of straight-
- * line network code, most of it in one warp at a time (about 16 cycles per
- * instruction in the solve, the right-hand side and the factorisation); no
- * memory traffic to speak of.  SYN64 against a thread per cell in
- * 256-thread blocks with the state in shared memory, B200: 65,536 cells FP32-LU 451 -> 245 ms, FP64 575 -> 515 ms, FP64 with
- * contraction 511 -> 428 ms; 3,001 cells FP32-LU 130 -> 25 ms, FP64 157 -> 38
- * ms; 64 cells FP64 121 -> 18 ms.
+ * Bound by one warp at a time: the others wait at a barrier (9.9 of the stall
+ * cycles per issued instruction over all warps) while one walks through its
+ * part of some 200 KB of straight-line network code, at about 16 cycles per
+ * instruction in the solve, the right-hand side and the factorisation;
+ * instruction fetch is 2.6 of the stall cycles, and no counter shows the
+ * working warp alone.  No memory traffic to speak of.  SYN64 against a thread
+ * per cell in 256-thread blocks with the state in shared memory, B200: 65,536
+ * cells FP32-LU 451 -> 245 ms, FP64 575 -> 515 ms, FP64 with contraction 511 ->
+ * 428 ms; 3,001 cells FP32-LU 130 -> 25 ms, FP64 157 -> 38 ms; 64 cells FP64
+ * 121 -> 18 ms.
  *
  * Barriers: every warp runs the same trip, and every condition around a
  * barrier is the same in all warps (ballots over state that all warps hold

@@ -5,10 +5,11 @@ different code.  Two ways to put them on the device at once:
 
 * ``fused=True``: one kernel launch (``odevec_solve_many``).  A
   multi-network kernel compiled for a set of variants (odevec_b200/build.py
-  MULTI_SETS) gives each job a share of the blocks in proportion to its cells;
-  a block whose job has no cells left takes cells of the other jobs, so the
-  networks share every SM for the whole launch.  The register budget is that
-  of the most demanding network in the set.
+  MULTI_SETS) runs each job as its network runs best alone, in blocks of 256
+  threads, one per SM.  A large network's cells get their blocks first, the
+  other jobs share the rest in proportion to their work; a block whose job has
+  no cells left takes cells of the other jobs, so the networks share every SM
+  for the whole launch.
 * ``fused=False``: one solve per network, each on its own stream forked from
   the capture stream, captured into a single CUDA graph; one replay (one
   cudaGraphLaunch) runs them concurrently, each with 1/k of the resident

@@ -256,7 +256,7 @@ class GpuBackend:
 
     def bytes_needed(self, r: Request) -> float:
         # state, times, workspace, status, statistics, and the solver's table
-        # of rate coefficients
+        # of rate coefficients (one, of this size: a request keeps its count)
         per_cell = (8 * (r.y0.shape[0] + 3 + self.S.workspace_doubles(r.network)
                          + self.S.network_info(r.network)["nrea"]) + 4 + 8 * 8)
         return float(per_cell * r.ncells)

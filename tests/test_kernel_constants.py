@@ -100,3 +100,51 @@ def test_no_rule_for_one_chip():
         if name.endswith((".cuh", ".cu", ".h", ".hpp")):
             code = re.sub(r"/\*.*?\*/|//[^\n]*", "", open(os.path.join(csrc, name)).read(), flags=re.S)
             assert not re.search(r"\b148\b", code), name
+
+
+def _exponents(pattern):
+    """[lo, hi) of the binary exponents that a range test of the kernel lets
+    through: upper word - (lo << 20) >= (span << 20) is outside"""
+    lo, span = map(int, re.search(pattern, open(CUH).read(), re.S).groups())
+    return lo - 1023, lo - 1023 + span
+
+
+RANGE = r"\((\d+)u << 20\) >= \((\d+)u << 20\)"
+
+
+@pytest.mark.parametrize("kind", ["weight", "pivot", "count"])
+def test_branch_free_ranges(kind):
+    """At the ends of the ranges that the kernel's own tests let through, the
+    branch-free reciprocals and quotients are correctly rounded and nothing
+    on the way under- or overflows."""
+    from fractions import Fraction as F
+    fma = lambda a, b, c: float(F(a) * F(b) + F(c))
+    values = lambda lo, hi: [math.ldexp(1.0 + m * 2.0 ** -52, e) for e in (lo, lo + 1, hi - 2, hi - 1)
+                             for m in (0, 1, 0x5555555555555, 0xaaaaaaaaaaaab, (1 << 52) - 2)]
+
+    def reciprocal(x):
+        want = float(1 / F(x))
+        for off in (-1.0, 1.0):
+            r = want * (1.0 + off * 2.0 ** -20)
+            for _ in range(3):
+                r = fma(fma(-x, r, 1.0), r, r)
+            assert r == want
+        return want
+
+    if kind == "weight":
+        for x in values(*_exponents(r"unsigned rcp_odd\(.*?" + RANGE)):
+            reciprocal(x)
+        return
+    if kind == "pivot":
+        divisors = values(*_exponents(r"ov_pivot\(const PivotRef& p\).*?" + RANGE))
+        xs = values(*_exponents(r"ov_divp\(T x, const PivotRef& p\).*?" + RANGE))
+    else:
+        divisors = [3.0, 5.0, 6.0, 7.0, 9.0, 12.0]
+        xs = values(*_exponents(r"double div_n\(double x\).*?" + RANGE))
+    for d in divisors:
+        r = reciprocal(d)
+        for x in xs:
+            q = x * r
+            q = fma(fma(-q, d, x), r, q)
+            q = fma(fma(-q, d, x), r, q)
+            assert q == x / d and abs(q) >= 2.0 ** -1022
