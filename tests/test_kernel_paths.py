@@ -477,3 +477,89 @@ def test_multi_block_limit(gpu_lib, n):
                 S.CloseOdevec(ode)
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", ["fp64_fma", "fp32_lu"])
+def test_block_kernel_forms_masked_and_resumed(gpu_lib, precision):
+    """The contracted forms with masked cells and CheckNegatives, then resumed:
+    the bits of a thread per cell (staging 15)."""
+    import torch
+    S = gpu_lib
+    wl = W.syn64(ncells=300, seed=15)
+    wl.t_stop[:] = 10.0 ** np.random.default_rng(3).uniform(-3.0, 3.0, 300)
+    mask = np.random.default_rng(4).random(300) > 0.2
+    got = []
+    for staging in (18, 15):
+        ode = _solver(S, wl, precision=precision, staging=staging, escalation=False, CheckNegatives=True)
+        try:
+            y, t, d = (torch.tensor(a, device="cuda") for a in (wl.y, wl.t0, wl.dt0))
+            ws = S.Workspace(ode, wl.ncells)
+            for k, resume in enumerate((False, True, "en_old")):
+                t, d = S.SolveODE(ode, t, d, torch.tensor(wl.t_stop * 2.0 ** k, device="cuda"), y, Mask=mask,
+                                  workspace=ws, resume=resume)
+            torch.cuda.synchronize()
+            got.append([a.cpu().numpy() for a in (y, t, d, ode.status, ode.stats)])
+        finally:
+            S.CloseOdevec(ode)
+    _same(got[0], got[1])
+
+
+def test_block_kernel_visit_order(gpu_lib):
+    """Cells of a large network visited longest span first, and in the given
+    order as ranges below the size from which there is an order: the same
+    bits."""
+    import torch
+    S = gpu_lib
+    n = 40000
+    wl = W.syn64(ncells=n, seed=16)
+    wl.t_stop[:] = 10.0 ** np.random.default_rng(5).uniform(-6.0, 0.0, n)
+    got = []
+    for ranges in ([(0, n)], [(0, 25000), (25000, n)]):
+        ode = _solver(S, wl)
+        try:
+            y, t, d, ts = (torch.tensor(a, device="cuda") for a in (wl.y, wl.t0, wl.dt0, wl.t_stop))
+            st = torch.zeros(n, dtype=torch.int32, device="cuda")
+            for c0, c1 in ranges:
+                S.SolveODERange(ode, c0, c1, t, d, ts, y, st)
+            torch.cuda.synchronize()
+            got.append([a.cpu().numpy() for a in (y, t, d, st)])
+        finally:
+            S.CloseOdevec(ode)
+    _same(got[0], got[1])
+
+
+def test_captured_solve_beyond_its_table(gpu_lib, oracle):
+    """A captured solve of more cells than the solver's rate table holds: the
+    solve kernel evaluates the rates."""
+    import torch
+    S = gpu_lib
+    a, b = W.primordial(ncells=4096, seed=34), W.primordial(ncells=9000, seed=35)
+    for wl in (a, b):
+        wl.t_stop[:] = 1e6
+    ode = _solver(S, b)
+    try:
+        _gpu(S, ode, a)
+        y, t, d, ts = (torch.tensor(v, device="cuda") for v in (b.y, b.t0, b.dt0, b.t_stop))
+        st = torch.zeros(b.ncells, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            S.SolveODERange(ode, 0, b.ncells, t, d, ts, y, st)
+        g.replay()
+        torch.cuda.synchronize()
+        _same([v.cpu().numpy() for v in (y, t, d, st)], _oracle(oracle, b)[:4])
+    finally:
+        S.CloseOdevec(ode)
+
+
+@pytest.mark.parametrize("group", [1, 32])
+def test_step_choice_ties(gpu_lib, oracle, group):
+    """Cells at rest, whose corrections are zero, so that all candidates of the
+    step-size choice are equal, beside ordinary ones."""
+    wl = W.rober(ncells=96, seed=17)
+    wl.y[:, 32:64] = np.array([0.0, 0.0, 1.0])[:, None]
+    ode = _solver(gpu_lib, wl, nvector=group)
+    try:
+        _same(_gpu(gpu_lib, ode, wl), _oracle(oracle, wl, group=group))
+    finally:
+        gpu_lib.CloseOdevec(ode)
